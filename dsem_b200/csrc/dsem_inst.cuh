@@ -3,6 +3,7 @@
 #include "dsem_launch.h"
 #include "dsem_stage.cuh"
 #include "dsem_vol_diag.cuh"
+#include "dsem_vol_mma.cuh"
 #include "dsem_lobatto.cuh"
 
 namespace dsem {
@@ -23,65 +24,77 @@ template <int G, bool DIAG, bool EV, int SAVE> static cudaError_t vol_one(const 
   return cudaGetLastError();
 }
 
-// diagonal metrics: k_vol_diag (two elements per SM at p = 8)
-template <int G, bool EV, int SAVE, int V = 0>
-static cudaError_t vol_diag_one(const VolArgs &a, int nel, cudaStream_t s) {
-  using C = VolDiagCfg<G, EV, SAVE, V>;
-  auto kern = k_vol_diag<G, EV, SAVE, V>;
+// diagonal metrics, p = 1, 2
+template <int G, bool EV, int SAVE> static cudaError_t vol_diag_one(const VolArgs &a, int nel, cudaStream_t s) {
+  using C = VolDiagCfg<G>;
+  auto kern = k_vol_diag<G, EV, SAVE>;
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = set_smem_once(kern, C::SMEM, attr);
   if (e != cudaSuccess) return e;
   if (nel <= 0) return cudaSuccess;
-  VolArgs b = a;
-  b.nel = nel;
-  kern<<<(nel + C::EPB - 1) / C::EPB, C::NT, C::SMEM, s>>>(b);
+  kern<<<nel, C::NT, C::SMEM, s>>>(a);
   return cudaGetLastError();
 }
 
-template <int G> size_t Launch<G>::vol_smem(bool diag, int mode) {
-  switch (mode) {
-    case VOL_SAVE: return diag ? VolDiagCfg<G, false, 1>::SMEM : VolCfg<G, false, false, 1>::SMEM;
-    case VOL_EV: return diag ? VolDiagCfg<G, true, 0>::SMEM : VolCfg<G, false, true, 0>::SMEM;
-    case VOL_EV_SAVE: return diag ? VolDiagCfg<G, true, 2>::SMEM : VolCfg<G, false, true, 2>::SMEM;
-    default: return diag ? VolDiagCfg<G, false, 0>::SMEM : VolCfg<G, false, false, 0>::SMEM;
-  }
-}
-template <int G> int Launch<G>::vol_threads(bool diag, int mode) {
-  (void)mode;
-  return diag ? VolDiagCfg<G, false, 0>::NT : VolCfg<G, false, false, 0>::NT;
+// diagonal metrics, p >= 3: line contractions on the FP64 matrix instruction
+template <int G, bool MU, int SAVE, int V = 0>
+static cudaError_t vol_mma_one(const VolArgs &a, int nel, cudaStream_t s) {
+  using C = MmaCfg<G, V>;
+  auto kern = k_vol_mma<G, MU, SAVE, V>;
+  static std::atomic<unsigned long long> attr{0};
+  cudaError_t e = set_smem_once(kern, C::SMEM, attr);
+  if (e != cudaSuccess) return e;
+  if (nel <= 0) return cudaSuccess;
+  kern<<<nel, C::NT, C::SMEM, s>>>(a);
+  return cudaGetLastError();
 }
 
-// launch-shape variants of k_vol_diag instantiated for this order (p = 4, 6, 8)
+// launch shapes of k_vol_mma instantiated for this order (p = 4, 6, 8)
 template <int G> int Launch<G>::vol_variants() { return (G == 5 || G == 7 || G == 9) ? VOL_VARIANTS : 1; }
-
-template <int G> int Launch<G>::vol_variant_threads(int v) {
-  switch (v) {
-    case 1: return VolDiagShape<G, 1>::NT;
-    case 2: return VolDiagShape<G, 2>::NT;
-    case 3: return VolDiagShape<G, 3>::NT;
-    case 4: return VolDiagShape<G, 4>::NT;
-    default: return VolDiagShape<G, 0>::NT;
-  }
-}
 
 template <int G>
 cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaStream_t s, int variant) {
-  if constexpr (G == 5 || G == 7 || G == 9) {  // variants of the diagonal kernel without entropy viscosity
-    if (diag && variant >= 1 && variant < VOL_VARIANTS && (mode == VOL_PLAIN || mode == VOL_SAVE)) {
-      const bool sv = mode == VOL_SAVE;
-      switch (variant) {
-        case 1: return sv ? vol_diag_one<G, false, 1, 1>(a, nel, s) : vol_diag_one<G, false, 0, 1>(a, nel, s);
-        case 2: return sv ? vol_diag_one<G, false, 1, 2>(a, nel, s) : vol_diag_one<G, false, 0, 2>(a, nel, s);
-        case 3: return sv ? vol_diag_one<G, false, 1, 3>(a, nel, s) : vol_diag_one<G, false, 0, 3>(a, nel, s);
-        default: return sv ? vol_diag_one<G, false, 1, 4>(a, nel, s) : vol_diag_one<G, false, 0, 4>(a, nel, s);
+  if (diag) {
+    if constexpr (G >= 4) {
+      const bool ev = mode == VOL_EV || mode == VOL_EV_SAVE;
+      VolArgs b = a;
+      if (!ev) b.muhg = nullptr;
+      constexpr int W = MMA_WIDE;
+      const bool wide = nel <= 148 * MmaShape<G, W>::MINB, sv = mode == VOL_SAVE;
+      if (ev || a.nuhg) {  // with a viscosity model: the default shape
+        switch (mode) {
+          case VOL_SAVE: return wide ? vol_mma_one<G, true, 1, W>(b, nel, s) : vol_mma_one<G, true, 1>(b, nel, s);
+          case VOL_EV_SAVE: return wide ? vol_mma_one<G, true, 2, W>(b, nel, s) : vol_mma_one<G, true, 2>(b, nel, s);
+          default: return wide ? vol_mma_one<G, true, 0, W>(b, nel, s) : vol_mma_one<G, true, 0>(b, nel, s);
+        }
+      }
+      if constexpr (G == 5 || G == 7 || G == 9) {
+        switch (variant) {
+          case 1: return sv ? vol_mma_one<G, false, 1, 1>(b, nel, s) : vol_mma_one<G, false, 0, 1>(b, nel, s);
+          case 2: return sv ? vol_mma_one<G, false, 1, 2>(b, nel, s) : vol_mma_one<G, false, 0, 2>(b, nel, s);
+          case 3: return sv ? vol_mma_one<G, false, 1, 3>(b, nel, s) : vol_mma_one<G, false, 0, 3>(b, nel, s);
+          case 4: return sv ? vol_mma_one<G, false, 1, 4>(b, nel, s) : vol_mma_one<G, false, 0, 4>(b, nel, s);
+        }
+      }
+      if (wide) return sv ? vol_mma_one<G, false, 1, W>(b, nel, s) : vol_mma_one<G, false, 0, W>(b, nel, s);
+      if constexpr (G == 5)  // p = 4: between the two, four warps per element
+        if (nel <= 148 * MmaShape<G, 3>::MINB)
+          return sv ? vol_mma_one<G, false, 1, 3>(b, nel, s) : vol_mma_one<G, false, 0, 3>(b, nel, s);
+      return sv ? vol_mma_one<G, false, 1>(b, nel, s) : vol_mma_one<G, false, 0>(b, nel, s);
+    } else {
+      switch (mode) {
+        case VOL_SAVE: return vol_diag_one<G, false, 1>(a, nel, s);
+        case VOL_EV: return vol_diag_one<G, true, 0>(a, nel, s);
+        case VOL_EV_SAVE: return vol_diag_one<G, true, 2>(a, nel, s);
+        default: return vol_diag_one<G, false, 0>(a, nel, s);
       }
     }
   }
   switch (mode) {
-    case VOL_SAVE: return diag ? vol_diag_one<G, false, 1>(a, nel, s) : vol_one<G, false, false, 1>(a, nel, s);
-    case VOL_EV: return diag ? vol_diag_one<G, true, 0>(a, nel, s) : vol_one<G, false, true, 0>(a, nel, s);
-    case VOL_EV_SAVE: return diag ? vol_diag_one<G, true, 2>(a, nel, s) : vol_one<G, false, true, 2>(a, nel, s);
-    default: return diag ? vol_diag_one<G, false, 0>(a, nel, s) : vol_one<G, false, false, 0>(a, nel, s);
+    case VOL_SAVE: return vol_one<G, false, false, 1>(a, nel, s);
+    case VOL_EV: return vol_one<G, false, true, 0>(a, nel, s);
+    case VOL_EV_SAVE: return vol_one<G, false, true, 2>(a, nel, s);
+    default: return vol_one<G, false, false, 0>(a, nel, s);
   }
 }
 

@@ -41,11 +41,8 @@ constexpr int VOL_VARIANTS = 5;
 
 template <int G> struct Launch {
   static cudaError_t set_ops(const double *host_ops, int n);  // copies the operator table to constant memory
-  static size_t vol_smem(bool diag, int mode);
-  static int vol_threads(bool diag, int mode);
   static cudaError_t vol(const VolArgs &a, int nel, bool diag, int mode, cudaStream_t s, int variant = 0);
   static int vol_variants();                // launch shapes available for this order (1 or VOL_VARIANTS)
-  static int vol_variant_threads(int v);    // threads per element of shape v
   static cudaError_t update(const UpdArgs &a, int nel, cudaStream_t s);
   static cudaError_t trace(const TraceArgs &a, int nel, cudaStream_t s);
   // Lobatto arrays of the stage kept in a.QLB; gradients rebuilt from them into a.EVB

@@ -962,7 +962,7 @@ __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, cons
         for (int v = 0; v < NV; ++v) VF[(fc - 1) * 5 * G2 + v * G2 + a + G * b] = r[v];
       } else {
         double fi[NV];
-        euler_flux(D, Q, rr, P.gamma, fi);
+        euler_flux(D, Q, rr, P.gm1, fi);
 #pragma unroll
         for (int v = 0; v < NV; ++v) CH[v * NLS + p] = gdiag * fi[v] - ddiv(r[v], P.re, P.r_re);
       }
@@ -986,7 +986,7 @@ __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, cons
 #pragma unroll
         for (int v = 0; v < NV; ++v) VF[(fc - 1) * 5 * G2 + v * G2 + a + G * b] = r[v];
       } else {
-        euler_fluxes3(Q, rr, P.gamma, f, g, h);
+        euler_fluxes3(Q, rr, P.gm1, f, g, h);
 #pragma unroll
         for (int v = 0; v < NV; ++v) CH[v * NLS + p] = (m0 * f[v] + m1 * g[v] + m2 * h[v]) - ddiv(r[v], P.re, P.r_re);
       }

@@ -1,12 +1,11 @@
 // dsem_vol_diag.cuh -- volume kernel for elements with diagonal metrics (the
-// axis-aligned hex elements of DSEM's boxes), sized for two CTAs per SM.
+// axis-aligned hex elements of DSEM's boxes) of the orders p = 1, 2; the orders
+// above run k_vol_mma (dsem_vol_mma.cuh).
 //
 // Same mathematics and the same floating-point evaluation order as k_vol
 // (Int_fluxes, Vis_Fluxes, Gauss_Deriv, update_interior:
 // fluxesH_newa.f90:221-355, Vis_Fluxes_new.f90:16-382, SolnDerivsc.f90:14-83,
-// updatea.f90:100-113), organised to keep about 107 KB of shared memory per
-// element at p = 8 so that two elements share an SM and hide each other's
-// latencies and barriers:
+// updatea.f90:100-113), one warp per element:
 //
 //  pass 1  one task per (direction D, field, line): the Lobatto line is built,
 //          differentiated and scaled by gmetg(D,D) in registers; the Gauss
@@ -27,46 +26,14 @@
 
 namespace dsem {
 
-// Launch shapes of k_vol_diag: threads per element (NT), the elements an SM
-// must hold at once (MINB, which sets the register budget), elements per block
-// (EPB: a block advances EPB elements one after another) and the Lobatto points
-// per flux task (PPT: 2, two points of a line sharing each gradient-line load, or
-// 1).  Variant 0 is the default; the autotuner (dsem_autotune) times variants
-// 1..4 against it for p = 4, 6, 8: 1 and 2 change the threads and register
-// budget, 3 takes two elements per block, 4 the other points-per-task.  Every
-// variant evaluates each value with the same FMA chain, so all give identical
-// results.
-#ifndef DSEM_VOL_DIAG_NT8
-#define DSEM_VOL_DIAG_NT8 192  // 2 CTAs x 6 warps per SM leave 168 registers per thread: no spills at p = 8
-#endif
-template <int G, int VV> struct VolDiagShape {
-  // p >= 7: 192 / 128 / 256 threads, two elements per SM (168 / 255 / 128 registers)
-  // p = 5, 6: 96 / 64 / 128 threads, four elements per SM (168 / 255 / 128 registers)
-  // p <= 4: 64 / 64 / 128 threads, eight / six / four elements per SM
-  // variants 3 and 4: the threads and register budget of variant 0
-  static constexpr int V = VV >= 3 ? 0 : VV;
-  static constexpr int NT = G >= 8 ? (V == 0 ? DSEM_VOL_DIAG_NT8 : (V == 1 ? 128 : 256))
-                                   : G >= 6 ? (V == 0 ? 96 : (V == 1 ? 64 : 128))
-                                            : G >= 4 ? (V == 2 ? 128 : 64) : 32;
-#ifdef DSEM_VOL_DIAG_MINB
-  static constexpr int MINB = V == 0 ? DSEM_VOL_DIAG_MINB : (G >= 8 ? 2 : (G >= 6 ? 4 : (V == 1 ? 6 : 4)));
-#else
-  static constexpr int MINB = G >= 8 ? 2 : (G >= 6 ? 4 : (G >= 4 ? (V == 0 ? 8 : (V == 1 ? 6 : 4)) : 16));
-#endif
-  static constexpr int EPB = VV == 3 ? 2 : 1;
-  // points per flux task: p = 8 (G = 9) two by default, lower orders one (measured: 12 % faster
-  // at p = 6); variant 4 takes the other
-  static constexpr int PPT_DEFAULT = G >= 8 ? 2 : 1;
-  static constexpr int PPT = VV == 4 ? 3 - PPT_DEFAULT : PPT_DEFAULT;
-};
-
-template <int G, bool EV, int SAVE, int V = 0> struct VolDiagCfg {
+// One warp per element: a line direction has 4 or 9 lines, too few for the 8-line
+// matrix tiles of k_vol_mma (at 32^3 elements of p = 2 that kernel takes 0.325 ms and
+// this one 0.184, at p = 1 0.165 and 0.077).
+template <int G> struct VolDiagCfg {
   static constexpr int L = G + 1, G2 = G * G, NG = G * G * G, NL = L * G * G;
-  static constexpr int NT = VolDiagShape<G, V>::NT;
-  static constexpr int NPT = (NG + NT - 1) / NT;       // Gauss points per thread (divergence)
-  static constexpr int MINB = VolDiagShape<G, V>::MINB;
-  static constexpr int EPB = VolDiagShape<G, V>::EPB, PPT = VolDiagShape<G, V>::PPT;
-  static constexpr int NGR = 12;                        // Gauss gradients of fields 0..3
+  static constexpr int NT = 32, MINB = 16;
+  static constexpr int NPT = (NG + NT - 1) / NT;  // Gauss points per thread (divergence)
+  static constexpr int NGR = 12;                  // Gauss gradients of fields 0..3
   static constexpr int NWORK = (6 * NL > 5 * NG) ? 6 * NL : 5 * NG;  // state (pass 1) / Lobatto arrays (pass 2)
   static constexpr size_t SMEM = sizeof(double) * (size_t)(NGR * NG + NWORK + 2 * G * L);
 };
@@ -197,7 +164,7 @@ __device__ __forceinline__ void vol_diag_point(int qi, int s, int a, int b, cons
     for (int v = 0; v < NV; ++v) VF[(fc - 1) * 5 * G2 + v * G2 + a + G * b] = r[v];
   } else {
     double fi[NV];
-    euler_flux(D, Q, rr, P.gamma, fi);
+    euler_flux(D, Q, rr, P.gm1, fi);
 #pragma unroll
     for (int v = 0; v < NV; ++v) LB[v * NL + qi] = gdiag * fi[v] - ddiv(r[v], P.re, P.r_re);
   }
@@ -205,13 +172,13 @@ __device__ __forceinline__ void vol_diag_point(int qi, int s, int a, int b, cons
 
 // Pass 2 along direction D: Lobatto arrays of grid D, fluxes at its points,
 // interior divergence accumulated into acc (the thread's Gauss points).
-template <int G, bool EV, int SAVE, int D, int V>
+template <int G, bool EV, int SAVE, int D>
 __device__ __forceinline__ void vol_diag_dir(const VolArgs &A, const Phys &P, const double *JQ, const double *jac,
                                              const double *QF, const double *gg, const double *gm, const double *muhg,
                                              const double *nuhg,
                                              const double *GR, double *LB, double *T4, const double *Bm,
                                              const double *Dm, double *VF, double *QTI, int tid, long long &t_ph_) {
-  using C = VolDiagCfg<G, EV, SAVE, V>;
+  using C = VolDiagCfg<G>;
   constexpr int L = G + 1, G2 = G * G, NG = G * G * G, NL = L * G * G, NT = C::NT, NPT = C::NPT;
   const int xs = D == 0 ? 1 : (D == 1 ? G : G2);
   const int ls = xs;  // Lobatto-grid stride along D (lstride)
@@ -255,67 +222,9 @@ __device__ __forceinline__ void vol_diag_dir(const VolArgs &A, const Phys &P, co
   for (int t = tid; t < 5 * G2; t += NT) a_task(4 - t / G2, t % G2);
   __syncthreads();
   PHASE_MARK(2 + 3 * (2 - D));
-  // (b) fluxes at the Lobatto points of grid D (Vis_Fluxes_new.f90:115-228, fluxesH_newa.f90:276-352),
-  // two points (s, s + NH) of one line per task so that both share the gradient loads.
-  // Whole rounds of tasks first; the tasks of a last, partial round are split into
-  // single points over twice as many threads, so that no thread computes two points
-  // more than another.
-  constexpr int NH = (L + 1) / 2;
-  constexpr int NTB = NH * G2, RB = NTB / NT, LEFTB = NTB - RB * NT;
-  constexpr bool SPLITB = LEFTB > 0 && 2 * LEFTB <= NT;
-  auto b_task = [&](int t) {
-    const int h = t / G2, ln = t - h * G2, a = ln % G, b = ln / G;
-    const int g0 = gbase<G>(D, a, b), l0 = lbase<G>(D, a, b);
-    const int s0 = h, s1 = h + NH;
-    const bool two = s1 < L;
-    const int s1c = two ? s1 : s0;
-    double br0[G], br1[G];
-#pragma unroll
-    for (int kk = 0; kk < G; ++kk) {
-      br0[kk] = Bm[s0 * G + kk];
-      br1[kk] = Bm[s1c * G + kk];
-    }
-    double c0[11], c1[11];
-#pragma unroll
-    for (int jf = 0; jf < 11; ++jf) {
-      if (jf == 4) {
-        c0[jf] = T4[l0 + s0 * ls];
-        c1[jf] = T4[l0 + s1c * ls];
-      } else {
-        const double *x = GR + diag_field(D, jf) * NG + g0;
-        double xv[G];
-#pragma unroll
-        for (int kk = 0; kk < G; ++kk) xv[kk] = x[kk * xs];
-        double a0 = br0[0] * xv[0], a1 = br1[0] * xv[0];
-#pragma unroll
-        for (int kk = 1; kk < G; ++kk) {
-          a0 = __fma_rn(br0[kk], xv[kk], a0);
-          a1 = __fma_rn(br1[kk], xv[kk], a1);
-        }
-        c0[jf] = a0;
-        c1[jf] = a1;
-      }
-    }
-    double mu0 = 0.0, mu1 = 0.0, nu0 = 0.0, nu1 = 0.0;
-    if (EV) {  // EV_Prolong (Prolong_gtol.f90:7-51)
-      mu0 = chain<G>(br0, muhg + g0, xs);
-      mu1 = chain<G>(br1, muhg + g0, xs);
-    }
-    const bool les = nuhg != nullptr;
-    if (les) {  // nut_prolong (staticSmag.f90:206-261): negative values clipped to 0
-      nu0 = chain<G>(br0, nuhg + g0, xs);
-      nu1 = chain<G>(br1, nuhg + g0, xs);
-      if (nu0 < 0.0) nu0 = 0.0;
-      if (nu1 < 0.0) nu1 = 0.0;
-    }
-    vol_diag_point<G, D>(l0 + s0 * ls, s0, a, b, c0, les, nu0, EV, mu0, P, gm, LB, VF);
-    if (two) vol_diag_point<G, D>(l0 + s1 * ls, s1, a, b, c1, les, nu1, EV, mu1, P, gm, LB, VF);
-  };
-  // one point of task t: s = h (which == 0) or h + NH, the same chains as b_task
-  auto b_point = [&](int t, int which) {
-    const int h = t / G2, ln = t - h * G2, a = ln % G, b = ln / G;
-    const int s0 = which ? h + NH : h;
-    if (s0 >= L) return;
+  // (b) fluxes at the Lobatto points of grid D (Vis_Fluxes_new.f90:115-228, fluxesH_newa.f90:276-352)
+  for (int t = tid; t < L * G2; t += NT) {
+    const int s0 = t / G2, ln = t - s0 * G2, a = ln % G, b = ln / G;
     const int g0 = gbase<G>(D, a, b), l0 = lbase<G>(D, a, b);
     double br0[G];
 #pragma unroll
@@ -331,14 +240,6 @@ __device__ __forceinline__ void vol_diag_dir(const VolArgs &A, const Phys &P, co
       if (nu0 < 0.0) nu0 = 0.0;
     }
     vol_diag_point<G, D>(l0 + s0 * ls, s0, a, b, c0, les, nu0, EV, mu0, P, gm, LB, VF);
-  };
-  if constexpr (C::PPT == 1) {  // one point per task
-    for (int u = tid; u < 2 * NTB; u += NT) b_point(u >> 1, u & 1);
-  } else if constexpr (SPLITB) {
-    for (int t = tid; t < RB * NT; t += NT) b_task(t);
-    if (tid < 2 * LEFTB) b_point(RB * NT + (tid >> 1), tid & 1);
-  } else {
-    for (int t = tid; t < NTB; t += NT) b_task(t);
   }
   // (c) interior divergence along D at this thread's Gauss points (updatea.f90:100-113),
   // summed over the directions in z, y, x order through the element's QTI slot; the
@@ -378,9 +279,9 @@ __device__ __forceinline__ void vol_diag_dir(const VolArgs &A, const Phys &P, co
 }
 
 // One element k of the volume kernel (its block's threads, shared memory sm).
-template <int G, bool EV, int SAVE, int V>
+template <int G, bool EV, int SAVE>
 __device__ __forceinline__ void vol_diag_element(const VolArgs &A, const int k, double *sm) {
-  using C = VolDiagCfg<G, EV, SAVE, V>;
+  using C = VolDiagCfg<G>;
   constexpr int L = G + 1, G2 = G * G, NG = G * G * G, NL = L * G * G, NT = C::NT;
   double *GR = sm;                  // [12][NG] Gauss gradients, field f*3 + direction
   double *WK = GR + C::NGR * NG;    // pass 1: state q [5][NG]; pass 2: LB [5][NL] + T4 [NL]
@@ -474,27 +375,16 @@ __device__ __forceinline__ void vol_diag_element(const VolArgs &A, const int k, 
 
   // ---- pass 2: z, y, x
   double *QTI = A.QTI + (long long)k * 5 * NG;
-  vol_diag_dir<G, EV, SAVE, 2, V>(A, P, JQ, jac, QF, gg, gm, muhg, nuhg, GR, LB, T4, Bm, Dm, VF, QTI, tid, t_ph_);
-  vol_diag_dir<G, EV, SAVE, 1, V>(A, P, JQ, jac, QF, gg, gm, muhg, nuhg, GR, LB, T4, Bm, Dm, VF, QTI, tid, t_ph_);
-  vol_diag_dir<G, EV, SAVE, 0, V>(A, P, JQ, jac, QF, gg, gm, muhg, nuhg, GR, LB, T4, Bm, Dm, VF, QTI, tid, t_ph_);
+  vol_diag_dir<G, EV, SAVE, 2>(A, P, JQ, jac, QF, gg, gm, muhg, nuhg, GR, LB, T4, Bm, Dm, VF, QTI, tid, t_ph_);
+  vol_diag_dir<G, EV, SAVE, 1>(A, P, JQ, jac, QF, gg, gm, muhg, nuhg, GR, LB, T4, Bm, Dm, VF, QTI, tid, t_ph_);
+  vol_diag_dir<G, EV, SAVE, 0>(A, P, JQ, jac, QF, gg, gm, muhg, nuhg, GR, LB, T4, Bm, Dm, VF, QTI, tid, t_ph_);
   PHASE_MARK(20);
 }
 
-template <int G, bool EV, int SAVE, int V = 0>
-__global__ void __launch_bounds__(VolDiagCfg<G, EV, SAVE, V>::NT, VolDiagCfg<G, EV, SAVE, V>::MINB)
-    k_vol_diag(VolArgs A) {
-  using C = VolDiagCfg<G, EV, SAVE, V>;
+template <int G, bool EV, int SAVE>
+__global__ void __launch_bounds__(VolDiagCfg<G>::NT, VolDiagCfg<G>::MINB) k_vol_diag(VolArgs A) {
   extern __shared__ double sm[];
-  if constexpr (C::EPB == 1) {
-    vol_diag_element<G, EV, SAVE, V>(A, blockIdx.x, sm);
-  } else {  // the block's elements one after another (each ends with a block barrier)
-#pragma unroll 1
-    for (int e = 0; e < C::EPB; ++e) {
-      const int k = blockIdx.x * C::EPB + e;
-      if (k >= A.nel) break;
-      vol_diag_element<G, EV, SAVE, V>(A, k, sm);
-    }
-  }
+  vol_diag_element<G, EV, SAVE>(A, blockIdx.x, sm);
 }
 
 }  // namespace dsem

@@ -1,0 +1,538 @@
+// dsem_vol_mma.cuh -- volume kernel for elements with diagonal metrics (the
+// axis-aligned hex elements of DSEM's boxes), p = 3..8, with the line
+// contractions on the FP64 matrix instruction (mma.sync m8n8k4 f64, DMMA).
+//
+// Same mathematics and the same floating-point evaluation order as k_vol
+// (Int_fluxes, Vis_Fluxes, Gauss_Deriv, update_interior:
+// fluxesH_newa.f90:221-355, Vis_Fluxes_new.f90:16-382, SolnDerivsc.f90:14-83,
+// updatea.f90:100-113): a DMMA runs the scalar contraction's FMA chain, in
+// increasing k from its accumulator, so the two kernels agree bit for bit.
+//
+// What bounds it: the FP64 pipe, which DMMA and DFMA share at 64 FMAs per clock
+// and SM.  A thread-per-point kernel reads every line value from shared memory once
+// per Lobatto point (24.7k shared-memory wavefronts per element at p = 8 against
+// 15.3k cycles of FP64 work) and passes Lobatto states and fluxes between phases
+// through it.  Here a warp takes 8 lines of a direction at once: rows of the
+// fragments are lines, columns their interior Lobatto points, so that every value
+// is loaded once per line, and
+//
+//  pass 1  per (direction, tile): the Lobatto lines of rho, rho u, rho v, rho w
+//          are interpolated, differentiated and scaled by gmetg(D,D) in registers;
+//          the Gauss gradients go to shared memory (12 fields);
+//  pass 2  per direction (z, y, x) and tile: the state and the 11 gradient fields
+//          the direction needs are interpolated; each lane then holds its line at
+//          s = 1+q and 5+q, evaluates both fluxes there, and its fluxes are already
+//          the A fragment of the divergence contraction (the columns of the
+//          interpolation are permuted so that they are).  No Lobatto array and no
+//          flux is written to memory.  Face points are separate tasks, one line per
+//          lane; the energy gradient is needed on its own grid only and is formed
+//          one direction ahead.
+// The divergence sums of the directions are added at L2 in the order z, y, x.
+//
+// Measured (22^3 elements of p = 8, the volume launch): 1.757 -> 1.127 ms; p = 7,
+// 20^3: 1.286 -> 0.492; p = 6, 24^3: 1.088 -> 0.745; p = 5, 24^3: 0.568 -> 0.526;
+// p = 4, 32^3: 0.716 -> 0.640; p = 3, 32^3: 0.371 -> 0.299.
+#pragma once
+#include "dsem_stage.cuh"
+
+namespace dsem {
+
+// D (8 x 8) += A (8 x 4) B (4 x 8).  Lane r*4+q holds A[r][q], B[q][r] and the
+// accumulators D[r][2q], D[r][2q+1].
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+// smallest plane stride >= G^2 congruent to 4 or 12 mod 16 doubles: the four
+// k-lanes of a fragment along z, and the four rows of one across z, then fall
+// into different banks
+__host__ __device__ constexpr int mma_plane(int G) {
+  int s = G * G;
+  while (s % 16 != 4 && s % 16 != 12) ++s;
+  return s;
+}
+
+// Launch shapes: warps per element (NW) and the elements an SM must hold at once
+// (MINB, which sets the register budget).  Variant 0 is the default; dsem_autotune times
+// 1..4 against it for p = 4, 6, 8.  Shared memory allows 2 elements per SM at p >= 7, 4 at
+// p = 6, 6 at p = 5 and 10 at p = 4.  Measured, ms of variants 0..4 (22^3 of p = 8, 24^3 of
+// p = 6, 32^3 of p = 4): 1.127 1.156 1.180 1.233 1.307; 0.745 0.762 0.946 0.739 0.854;
+// 0.640 0.708 0.644 0.700 0.671.  Every shape evaluates each value with the same chain.
+// MMA_WIDE: the shape of variant 0 for launches of at most 148 * MINB elements, which do
+// not fill the GPU: more warps work on one element, and its latency is the launch's.
+// Measured against variant 1's or 0's shape, us: 4^3 elements of p = 8 23.8 (8 warps: 27),
+// p = 6 15.6 (3 warps: 24.7), p = 4 10.4 (2 warps: 16.5); p = 4 at 512 elements, which
+// variant 3 still holds at once, 16.5 with it (2 warps: 19.6).
+constexpr int MMA_WIDE = 5;
+template <int G, int V> struct MmaShape {
+  static constexpr bool W = V == MMA_WIDE;
+  static constexpr int NW = G >= 8 ? (W ? 16 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 7 : (V == 3 ? 5 : 4)))))
+                          : G >= 6 ? (W ? (G == 7 ? 12 : 8) : (V == 0 ? 4 : (V == 1 ? 3 : (V == 2 ? 2 : (V == 3 ? 5 : 6)))))
+                          : G == 5 ? (W ? 8 : (V <= 2 ? 2 : (V == 3 ? 4 : 3)))
+                                   : (W ? 4 : 2);
+  static constexpr int MINB = G >= 8 ? (W ? 1 : 2)
+                            : G >= 6 ? (W ? (G == 7 ? 1 : 2) : (V == 3 ? 3 : (V == 4 ? 2 : 4)))
+                            : G == 5 ? (W ? 2 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 10 : (V == 3 ? 4 : 5)))))
+                                     : (W ? 4 : 8);
+};
+
+template <int G, int V> struct MmaCfg {
+  static constexpr int L = G + 1, G2 = G * G, NG = G * G * G, NL = L * G * G;
+  static constexpr int PS = mma_plane(G), FS = G * PS;  // padded plane and field strides
+  static constexpr int NS = G - 1;                      // interior Lobatto points s = 1..NS
+  static constexpr int NI = NS > 4 ? 2 : 1;             // interior points per lane: s = 1+q, 5+q
+  static constexpr int KF = G / 4, KR = G % 4;          // full k-steps and remaining k of a Gauss contraction
+  static constexpr int KM = KR == 3 ? KF + 1 : KF;      // k-steps on the matrix unit (a remainder of 3 padded)
+  static constexpr int KS = KR == 3 ? 0 : KR;           // k on scalar FMAs
+  static constexpr int NTILE = (G2 + 7) / 8;            // tiles of 8 lines per direction
+  static constexpr int NLW = (G2 + 31) / 32;            // warps of one line per lane
+  static constexpr int NW = MmaShape<G, V>::NW, NT = 32 * NW;
+  static constexpr int MINB = MmaShape<G, V>::MINB;
+  static constexpr int NF = 19;  // shared fields: state 5, gradients of fields 0..3 12, energy gradient 2 buffers
+  static constexpr size_t SMEM = sizeof(double) * (size_t)(NF * FS) + 16;
+};
+
+// Operator entries of one lane (fragment column n = lane / 4, k = q = lane % 4):
+// column n of the interpolation is s = 1 + n/2 + 4 (n&1), column n of the
+// divergence Gauss point n/2 + 4 (n&1), so that lane q of a quad owns s = 1+q,
+// 5+q and Gauss points q, 4+q.
+template <int G, int V> struct MmaOps {
+  using C = MmaCfg<G, V>;
+  double bm[C::KM > 0 ? C::KM : 1], b0[C::KS > 0 ? C::KS : 1], b1[C::KS > 0 ? C::KS : 1], dm[2], d8[2];
+  double dlo[2], dhi[2];  // first and last column of dmx at Gauss points q, 4+q
+  __device__ __forceinline__ void load() {
+    const int q = threadIdx.x & 3, n = (threadIdx.x & 31) >> 2, kn = (n >> 1) + 4 * (n & 1), sn = 1 + kn;
+#pragma unroll
+    for (int j = 0; j < C::KM; ++j) bm[j] = (sn <= C::NS && 4 * j + q < G) ? Op<G>::B(sn, 4 * j + q) : 0.0;
+#pragma unroll
+    for (int k = 0; k < C::KS; ++k) {
+      b0[k] = 1 + q <= C::NS ? Op<G>::B(1 + q, 4 * C::KF + k) : 0.0;
+      b1[k] = 5 + q <= C::NS ? Op<G>::B(5 + q, 4 * C::KF + k) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < C::NI; ++j) {
+      const int s = 1 + 4 * j + q;
+      dm[j] = (kn < G && s <= C::NS) ? Op<G>::D(kn, s) : 0.0;
+      d8[j] = (G == 9 && n == 0 && s <= C::NS) ? Op<G>::D(G - 1, s) : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      dlo[i] = 4 * i + q < G ? Op<G>::D(4 * i + q, 0) : 0.0;
+      dhi[i] = 4 * i + q < G ? Op<G>::D(4 * i + q, G) : 0.0;
+    }
+  }
+};
+
+// line (a, b) of row r: across z for direction x (no bank conflicts), else x fastest
+template <int G, int D> __device__ __forceinline__ void mma_line(int r, int &a, int &b) {
+  if (D == 0) {
+    b = r % G;
+    a = r / G;
+  } else {
+    a = r % G;
+    b = r / G;
+  }
+}
+template <int G, int D> __device__ __forceinline__ int mma_base(int a, int b) {  // padded Gauss layout
+  constexpr int PS = mma_plane(G);
+  return D == 0 ? G * a + PS * b : (D == 1 ? a + PS * b : a + G * b);
+}
+template <int G, int D> __device__ __forceinline__ constexpr int mma_stride() {
+  return D == 0 ? 1 : (D == 1 ? G : mma_plane(G));
+}
+
+// Viscous flux of direction D times gdiag into r from the point's state and its
+// 11 interpolated gradient fields (diag_field order).
+template <int D>
+__device__ __forceinline__ void mma_vis(const double *Q, double rr, const double *c, double amu, double gdiag,
+                                        const Phys &P, double *r) {
+  double Qx[NV], Qy[NV], Qz[NV], fl[NV];
+  if (D == 0) {
+    Qx[0] = c[0]; Qx[1] = c[1]; Qx[2] = c[2]; Qx[3] = c[3]; Qx[4] = c[4];
+    Qy[0] = c[5]; Qy[1] = c[6]; Qy[2] = c[7]; Qy[3] = 0.0; Qy[4] = 0.0;
+    Qz[0] = c[8]; Qz[1] = c[9]; Qz[3] = c[10]; Qz[2] = 0.0; Qz[4] = 0.0;
+    vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, fl);
+  } else if (D == 1) {
+    Qy[0] = c[0]; Qy[1] = c[1]; Qy[2] = c[2]; Qy[3] = c[3]; Qy[4] = c[4];
+    Qx[0] = c[5]; Qx[1] = c[6]; Qx[2] = c[7]; Qx[3] = 0.0; Qx[4] = 0.0;
+    Qz[0] = c[8]; Qz[2] = c[9]; Qz[3] = c[10]; Qz[1] = 0.0; Qz[4] = 0.0;
+    vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, fl);
+  } else {
+    Qz[0] = c[0]; Qz[1] = c[1]; Qz[2] = c[2]; Qz[3] = c[3]; Qz[4] = c[4];
+    Qx[0] = c[5]; Qx[1] = c[6]; Qx[3] = c[7]; Qx[2] = 0.0; Qx[4] = 0.0;
+    Qy[0] = c[8]; Qy[2] = c[9]; Qy[3] = c[10]; Qy[1] = 0.0; Qy[4] = 0.0;
+    vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, fl);
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) r[v] = gdiag * fl[v];
+}
+
+// Interpolation to the interior points of a tile's 8 lines: lane r*4+q gets the
+// values of line r at s = 1+q (c0) and 5+q (c1).  x: the lane's line at k = q;
+// xl: the lane's line at k = 0.
+template <int G, int V, int S>
+__device__ __forceinline__ void mma_interp(const double *x, const double *xl, const MmaOps<G, V> &O, double &c0,
+                                           double &c1) {
+  using C = MmaCfg<G, V>;
+  c0 = 0.0;
+  c1 = 0.0;
+#pragma unroll
+  for (int j = 0; j < C::KF; ++j) dmma(c0, c1, x[4 * j * S], O.bm[j]);
+  if constexpr (C::KM > C::KF) {  // padded k: the line's last value against a zero coefficient
+    const int q = threadIdx.x & 3;
+    dmma(c0, c1, xl[(4 * C::KF + (q < C::KR ? q : C::KR - 1)) * S], O.bm[C::KF]);
+  }
+#pragma unroll
+  for (int k = 0; k < C::KS; ++k) {
+    const double xv = xl[(4 * C::KF + k) * S];
+    c0 = __fma_rn(O.b0[k], xv, c0);
+    if (C::NI == 2) c1 = __fma_rn(O.b1[k], xv, c1);
+  }
+}
+
+// Gradients along D of NV1 fields (state sq, from field v0) on a tile's 8 lines: the Lobatto
+// lines are interpolated, differentiated and scaled by gmetg(D,D) in registers
+// (k_vol's chains); field i goes to out + i * os.
+template <int G, int V, int D, int NV1>
+__device__ __forceinline__ void mma_grad(int t, const MmaOps<G, V> &O, const double *sq, int v0, const double *QF,
+                                         const double *gg, double *out, int os) {
+  using C = MmaCfg<G, V>;
+  constexpr int L = C::L, G2 = C::G2, NG = C::NG, FS = C::FS;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int lane = threadIdx.x & 31, q = lane & 3, n = lane >> 2;
+  const bool row = t * 8 + n < G2;
+  int a, b;
+  mma_line<G, D>(row ? t * 8 + n : G2 - 1, a, b);
+  const int pl = mma_base<G, D>(a, b), pq = pl + q * S;
+  const double *m = gg + D * NG + gbase<G>(D, a, b) + q * xs;
+  const double m0 = q < G ? __ldg(m) : 0.0, m1 = 4 + q < G ? __ldg(m + 4 * xs) : 0.0;
+  const double m2 = G == 9 && q == 0 ? __ldg(m + 8 * xs) : 0.0;
+  const double *flo = QF + ((face_lo(D) - 1) * 5 + v0) * G2 + a + G * b;
+  const double *fhi = QF + ((face_hi(D) - 1) * 5 + v0) * G2 + a + G * b;
+  double y0[NV1], y1[NV1];
+#pragma unroll
+  for (int i = 0; i < NV1; ++i) {
+    y0[i] = __ldg(flo + i * G2);
+    y1[i] = __ldg(fhi + i * G2);
+  }
+#pragma unroll
+  for (int i = 0; i < NV1; ++i) {
+    double c[2];
+    mma_interp<G, V, S>(sq + (v0 + i) * FS + pq, sq + (v0 + i) * FS + pl, O, c[0], c[1]);
+    double e0 = O.dlo[0] * y0[i], e1 = O.dlo[1] * y0[i], g0 = Op<G>::D(G - 1, 0) * y0[i], g1 = 0.0;
+#pragma unroll
+    for (int j = 0; j < C::NI; ++j) {
+      dmma(e0, e1, c[j], O.dm[j]);
+      if (G == 9) dmma(g0, g1, c[j], O.d8[j]);
+    }
+    e0 = __fma_rn(O.dhi[0], y1[i], e0);
+    e1 = __fma_rn(O.dhi[1], y1[i], e1);
+    g0 = __fma_rn(Op<G>::D(G - 1, L - 1), y1[i], g0);
+    double *o = out + i * os + pq;
+    if (row) {
+      if (q < G) o[0] = m0 * e0;
+      if (4 + q < G) o[4 * S] = m1 * e1;
+      if (G == 9 && q == 0) o[8 * S] = m2 * g0;
+    }
+  }
+}
+
+// Adds a direction's part of the divergence to its QTI slot, in the order z (a store), y, x:
+// the block barrier between the directions orders the additions, and a reduction at L2
+// (rounded to nearest, like the plain sum) needs no load in the tile.
+template <int D> __device__ __forceinline__ void mma_add(double *o, double x) {
+  if (D == 2)
+    *o = x;
+  else
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(x) : "memory");
+}
+
+// One tile of direction D: 8 lines, all their interior Lobatto points.  The
+// state and gradient fields are interpolated, both fluxes evaluated and the
+// interior divergence contracted without leaving the warp's registers.
+template <int G, bool MU, int V, int D>
+__device__ __forceinline__ void mma_tile(int t, const MmaOps<G, V> &O, const Phys &P, const double *sq, const double *GR, const double *E4,
+                                         const double *gm, const double *muhg, const double *nuhg, double *QTI) {
+  using C = MmaCfg<G, V>;
+  constexpr int G2 = C::G2, NG = C::NG, NL = C::NL, FS = C::FS;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int lane = threadIdx.x & 31, q = lane & 3, n = lane >> 2;
+  const bool row = t * 8 + n < G2;
+  int a, b;
+  mma_line<G, D>(row ? t * 8 + n : G2 - 1, a, b);
+  const int pl = mma_base<G, D>(a, b), pq = pl + q * S;
+  const int l0 = lbase<G>(D, a, b) + (1 + q) * xs;  // Lobatto point s = 1 + q
+  double Q[2][NV], c[2][11], gd[2], nu[2] = {0.0, 0.0}, mu[2] = {0.0, 0.0};
+  gd[0] = 1 + q <= C::NS ? __ldg(gm + D * NL + l0) : 0.0;
+  gd[1] = (C::NI == 2 && 5 + q <= C::NS) ? __ldg(gm + D * NL + l0 + 4 * xs) : 0.0;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) mma_interp<G, V, S>(sq + v * FS + pq, sq + v * FS + pl, O, Q[0][v], Q[1][v]);
+#pragma unroll
+  for (int f = 0; f < 11; ++f) {
+    const double *x = f == 4 ? E4 : GR + diag_field(D, f) * FS;
+    mma_interp<G, V, S>(x + pq, x + pl, O, c[0][f], c[1][f]);
+  }
+  const bool ev = MU && muhg != nullptr, les = MU && nuhg != nullptr;
+  if (ev) {  // EV_Prolong (Prolong_gtol.f90:7-51)
+    const double *x = muhg + gbase<G>(D, a, b);
+    mma_interp<G, V, xs>(x + q * xs, x, O, mu[0], mu[1]);
+  }
+  if (les) {  // nut_prolong (staticSmag.f90:206-261): negative values clipped to 0
+    const double *x = nuhg + gbase<G>(D, a, b);
+    mma_interp<G, V, xs>(x + q * xs, x, O, nu[0], nu[1]);
+    if (nu[0] < 0.0) nu[0] = 0.0;
+    if (nu[1] < 0.0) nu[1] = 0.0;
+  }
+  double f[2][NV];
+#pragma unroll
+  for (int i = 0; i < C::NI; ++i) {
+    double amu = 1.0;  // Vis_Fluxes_new.f90:123-125
+    if (les) amu = amu + nu[i] * Q[i][0];
+    if (ev) amu = amu + mu[i];
+    const double rr = 1.0 / Q[i][0];
+    double r[NV], fi[NV];
+    mma_vis<D>(Q[i], rr, c[i], amu, gd[i], P, r);
+    euler_flux(D, Q[i], rr, P.gm1, fi);
+    const bool in = (i == 0 ? 1 : 5) + q <= C::NS;  // padded points contribute exact zeros
+#pragma unroll
+    for (int v = 0; v < NV; ++v) f[i][v] = in ? gd[i] * fi[v] - ddiv(r[v], P.re, P.r_re) : 0.0;
+  }
+  // interior divergence along D (updatea.f90:100-113), k = s - 1: lane r*4+q gets line r at
+  // Gauss points q and 4+q; the ninth Gauss point of G = 9 is a column of its own (q = 0)
+  double *qt = QTI + gbase<G>(D, a, b);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    double e0 = 0.0, e1 = 0.0, g0 = 0.0, g1 = 0.0;
+#pragma unroll
+    for (int j = 0; j < C::NI; ++j) {
+      dmma(e0, e1, f[j][v], O.dm[j]);
+      if (G == 9) dmma(g0, g1, f[j][v], O.d8[j]);
+    }
+    if (row) {
+      double *o = qt + v * NG + q * xs;
+      if (q < G) mma_add<D>(o, e0);
+      if (4 + q < G) mma_add<D>(o + 4 * xs, e1);
+      if (G == 9 && q == 0) mma_add<D>(o + 8 * xs, g0);
+    }
+  }
+}
+
+// Viscous fluxes at both face points of one line of direction D per lane
+// (Vis_Fluxes_new.f90:115-228), written to VF.
+template <int G, bool MU, int V, int D>
+__device__ __forceinline__ void mma_faces(int ln, const Phys &P, const double *QF, const double *GR, const double *E4,
+                                          const double *gm, const double *muhg, const double *nuhg, double *VF) {
+  using C = MmaCfg<G, V>;
+  constexpr int L = C::L, G2 = C::G2, NL = C::NL, FS = C::FS;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int a = ln % G, b = ln / G;
+  const int pl = mma_base<G, D>(a, b);
+  const double *qlo = QF + (face_lo(D) - 1) * 5 * G2 + ln, *qhi = QF + (face_hi(D) - 1) * 5 * G2 + ln;
+  const double *g = gm + D * NL + lbase<G>(D, a, b);
+  double Q[2][NV], gd[2] = {__ldg(g), __ldg(g + (L - 1) * xs)};
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    Q[0][v] = __ldg(qlo + v * G2);
+    Q[1][v] = __ldg(qhi + v * G2);
+  }
+  double c[2][11], nu[2] = {0.0, 0.0}, mu[2] = {0.0, 0.0};
+  auto ends = [&](const double *x, int st, double &lo, double &hi) {
+    const double x0 = x[0];
+    lo = Op<G>::B(0, 0) * x0;
+    hi = Op<G>::B(L - 1, 0) * x0;
+#pragma unroll
+    for (int k = 1; k < G; ++k) {
+      const double xv = x[k * st];
+      lo = __fma_rn(Op<G>::B(0, k), xv, lo);
+      hi = __fma_rn(Op<G>::B(L - 1, k), xv, hi);
+    }
+  };
+#pragma unroll
+  for (int f = 0; f < 11; ++f) ends((f == 4 ? E4 : GR + diag_field(D, f) * FS) + pl, S, c[0][f], c[1][f]);
+  const bool ev = MU && muhg != nullptr, les = MU && nuhg != nullptr;
+  if (ev) ends(muhg + gbase<G>(D, a, b), xs, mu[0], mu[1]);
+  if (les) {
+    ends(nuhg + gbase<G>(D, a, b), xs, nu[0], nu[1]);
+    if (nu[0] < 0.0) nu[0] = 0.0;
+    if (nu[1] < 0.0) nu[1] = 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    double r[NV];
+    double amu = 1.0;
+    if (les) amu = amu + nu[i] * Q[i][0];
+    if (ev) amu = amu + mu[i];
+    mma_vis<D>(Q[i], 1.0 / Q[i][0], c[i], amu, gd[i], P, r);
+    double *o = VF + ((i ? face_hi(D) : face_lo(D)) - 1) * 5 * G2 + ln;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) o[v * G2] = r[v];
+  }
+}
+
+// Phase of direction D: its face points, the energy gradient of the next
+// direction (z, y, x), and its tiles, drawn by the warps from one list.
+template <int G, bool MU, int V, int D>
+__device__ __forceinline__ void mma_phase(int *next, const MmaOps<G, V> &O, const Phys &P, const double *sq, const double *GR, const double *E4,
+                                          double *E4n, const double *QF, const double *gg, const double *gm,
+                                          const double *muhg, const double *nuhg, double *VF, double *QTI) {
+  using C = MmaCfg<G, V>;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = C::NW - 1 - w; i < C::NLW; i += C::NW)
+    if (i * 32 + lane < C::G2) mma_faces<G, MU, V, D>(i * 32 + lane, P, QF, GR, E4, gm, muhg, nuhg, VF);
+  __syncwarp();
+  for (;;) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(next, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= (D > 0 ? 2 : 1) * C::NTILE) break;
+    if (t >= C::NTILE)  // the next direction's energy gradient (needed on grid D only)
+      mma_grad<G, V, (D > 0 ? D - 1 : 0), 1>(t - C::NTILE, O, sq, 4, QF, gg, E4n, 0);
+    else
+      mma_tile<G, MU, V, D>(t, O, P, sq, GR, E4, gm, muhg, nuhg, QTI);
+  }
+}
+
+// Temperature gradient along D (EV runs, SAVE == 2): the five Lobatto lines, the
+// temperature on them (RHS.f90:66-83), its derivative scaled by gmetg(D,D).
+template <int G, int V, int D>
+__device__ __forceinline__ void mma_tgrad(int ln, const double *sq, const double *QF, const double *gg, double *EVB,
+                                          double gamma) {
+  constexpr int L = G + 1, G2 = G * G, NG = G * G * G, FS = MmaCfg<G, V>::FS;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int a = ln % G, b = ln / G;
+  const int pl = mma_base<G, D>(a, b), p0 = gbase<G>(D, a, b);
+  double y[5][L];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    double x[G];
+#pragma unroll
+    for (int kk = 0; kk < G; ++kk) x[kk] = sq[v * FS + pl + kk * S];
+    y[v][0] = __ldg(QF + (face_lo(D) - 1) * 5 * G2 + v * G2 + ln);
+    y[v][L - 1] = __ldg(QF + (face_hi(D) - 1) * 5 * G2 + v * G2 + ln);
+#pragma unroll
+    for (int s = 1; s < L - 1; ++s) {
+      double acc = Op<G>::B(s, 0) * x[0];
+#pragma unroll
+      for (int kk = 1; kk < G; ++kk) acc = __fma_rn(Op<G>::B(s, kk), x[kk], acc);
+      y[v][s] = acc;
+    }
+  }
+  double T[L];
+#pragma unroll
+  for (int s = 0; s < L; ++s) {
+    const double q1 = y[0][s], q2 = y[1][s], q3 = y[2][s], q4 = y[3][s], q5 = y[4][s];
+    const double r1 = 1.0 / q1, u = ddiv(q2, q1, r1), v = ddiv(q3, q1, r1), w = ddiv(q4, q1, r1);
+    const double Pp = (gamma - 1.0) * (q5 - 0.5 * q1 * (u * u + v * v + w * w));
+    T[s] = ddiv(Pp * gamma, q1, r1);
+  }
+#pragma unroll
+  for (int kk = 0; kk < G; ++kk) {
+    double acc = Op<G>::D(kk, 0) * T[0];
+#pragma unroll
+    for (int s = 1; s < L; ++s) acc = __fma_rn(Op<G>::D(kk, s), T[s], acc);
+    EVB[(12 + D) * NG + p0 + kk * xs] = gg[D * NG + p0 + kk * xs] * acc;
+  }
+}
+
+template <int G, bool MU, int SAVE, int V = 0>
+__global__ void __launch_bounds__(MmaCfg<G, V>::NT, MmaCfg<G, V>::MINB) k_vol_mma(VolArgs A) {
+  using C = MmaCfg<G, V>;
+  constexpr int G2 = C::G2, NG = C::NG, NL = C::NL, NT = C::NT, FS = C::FS, PS = C::PS;
+  extern __shared__ double sm[];
+  double *sq = sm;              // [5] state
+  double *GR = sq + 5 * FS;     // [12] Gauss gradients, field v*3 + direction
+  double *E0 = GR + 12 * FS;    // energy gradient along z, then along x
+  double *E1 = E0 + FS;         // energy gradient along y
+  int *next = reinterpret_cast<int *>(E1 + FS);  // [3] work lists of the phases
+  const int tid = threadIdx.x, k = blockIdx.x;
+  const double *JQ = A.JQ + (long long)k * A.sq;
+  const double *jac = A.jac + (long long)k * NG;
+  const double *QF = A.QF + (long long)k * 30 * G2;
+  double *VF = A.VF + (long long)k * 30 * G2;
+  const double *gg = A.gg + (long long)k * 3 * NG;
+  const double *gm = A.gm + (long long)k * 3 * NL;
+  const double *muhg = MU && A.muhg ? A.muhg + (long long)k * NG : nullptr;  // viscosity models in use
+  const double *nuhg = MU && A.nuhg ? A.nuhg + (long long)k * NG : nullptr;
+  double *EVB = SAVE ? A.EVB + (long long)k * 15 * NG : nullptr;
+  double *QTI = A.QTI + (long long)k * 5 * NG;
+  Phys P = A.P;
+  if (A.rec) {  // per-case Reynolds number
+    const int cs = A.ecase[k];
+    P.re = A.rec[2 * cs];
+    P.r_re = A.rec[2 * cs + 1];
+  }
+  if (tid == 0) {
+    prefetch_l2_bulk(gg, 3 * NG);
+    prefetch_l2_bulk(gm, 3 * NL);
+    prefetch_l2_bulk(QF, 30 * G2);
+    if (muhg) prefetch_l2_bulk(muhg, NG);
+    if (nuhg) prefetch_l2_bulk(nuhg, NG);
+  }
+  if (tid < 3) next[tid] = 0;
+  long long t_ph_ = 0;
+#ifdef DSEM_PHASE_TIMING
+  t_ph_ = clock64();
+#endif
+  // Q*jacob (fluxesH_newa.f90:262-272), all of a thread's loads in flight at once
+  {
+    constexpr int NQ = (5 * NG + NT - 1) / NT;
+    double qv[NQ], jv[NQ];
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      const int i = tid + j * NT;
+      if (i < 5 * NG) {
+        qv[j] = JQ[i];
+        jv[j] = jac[i % NG];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      const int i = tid + j * NT;
+      if (i < 5 * NG) sq[i / G2 * PS + i % G2] = qv[j] * jv[j];
+    }
+  }
+  __syncthreads();
+  PHASE_MARK(0);
+  MmaOps<G, V> O;
+  O.load();
+  // pass 1: Gauss gradients of fields 0..3 (and of the energy along z), a tile of lines per task
+  for (int t = tid >> 5; t < 3 * C::NTILE; t += C::NW) {
+    if (t < C::NTILE) {
+      mma_grad<G, V, 2, 4>(t, O, sq, 0, QF, gg, GR + 2 * FS, 3 * FS);
+      mma_grad<G, V, 2, 1>(t, O, sq, 4, QF, gg, E0, 0);
+    } else if (t < 2 * C::NTILE) {
+      mma_grad<G, V, 1, 4>(t - C::NTILE, O, sq, 0, QF, gg, GR + FS, 3 * FS);
+    } else {
+      mma_grad<G, V, 0, 4>(t - 2 * C::NTILE, O, sq, 0, QF, gg, GR, 3 * FS);
+    }
+  }
+  if (SAVE == 2) {
+    for (int t = tid; t < 3 * G2; t += NT) {
+      const int D = t / G2, ln = t - D * G2;
+      if (D == 0)
+        mma_tgrad<G, V, 0>(ln, sq, QF, gg, EVB, P.gamma);
+      else if (D == 1)
+        mma_tgrad<G, V, 1>(ln, sq, QF, gg, EVB, P.gamma);
+      else
+        mma_tgrad<G, V, 2>(ln, sq, QF, gg, EVB, P.gamma);
+    }
+  }
+  __syncthreads();
+  PHASE_MARK(1);
+  if (SAVE) {
+    for (int i = tid; i < 12 * NG; i += NT) EVB[i] = GR[i / G2 * PS + i % G2];
+  }
+  // pass 2: z, y, x
+  mma_phase<G, MU, V, 2>(next + 0, O, P, sq, GR, E0, E1, QF, gg, gm, muhg, nuhg, VF, QTI);
+  __syncthreads();
+  PHASE_MARK(2);
+  mma_phase<G, MU, V, 1>(next + 1, O, P, sq, GR, E1, E0, QF, gg, gm, muhg, nuhg, VF, QTI);
+  __syncthreads();
+  PHASE_MARK(3);
+  mma_phase<G, MU, V, 0>(next + 2, O, P, sq, GR, E0, E1, QF, gg, gm, muhg, nuhg, VF, QTI);
+  PHASE_MARK(4);
+}
+
+}  // namespace dsem
