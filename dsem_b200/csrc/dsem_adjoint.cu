@@ -62,14 +62,42 @@ struct AdjBuf {
   double *evb_prev = nullptr;
   double *lrb = nullptr;  // boundary faces: per boundary point, dJ/d(1/Re) of the external viscous flux
   double *volscr = nullptr;  // p = 7, 8: the volume adjoint's per element scratch (VolAdjCfg::SCR)
+  // Device memory from the context's pool, in stream order: cudaMalloc and cudaFree of these
+  // buffers took 11 ms and more of a 44 ms call (8^3 elements of p = 6, 30 steps) and up to
+  // 170 ms when the driver unmapped them; from the pool a repeated call finds them mapped.
+  dsem_ctx *c = nullptr;
+  cudaError_t alloc(double **p, size_t bytes) {
+    return cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, c->adj_pool, c->st);
+  }
+  void release(double *&p) {
+    if (p) cudaFreeAsync(p, c->st);
+    p = nullptr;
+  }
   ~AdjBuf() {
-    for (double *p : {lq, lg, ljq, qfr, lff, lvf, lqf, lqr, lrp, lr, q0, stages, traces, lmuhg, levb, evb0,
-                      eps_part, evbw, evb_prev, lrb, volscr})
-      cudaFree(p);
-    for (double *p : slots) cudaFree(p);
-    for (double *p : slot_evb) cudaFree(p);
+    for (double **p : {&lq, &lg, &ljq, &qfr, &lff, &lvf, &lqf, &lqr, &lrp, &lr, &q0, &stages, &traces, &lmuhg, &levb,
+                       &evb0, &eps_part, &evbw, &evb_prev, &lrb, &volscr})
+      release(*p);
+    for (double *&p : slots) release(p);
+    for (double *&p : slot_evb) release(p);
+    if (c) cudaStreamSynchronize(c->st);  // what the pool does not keep is given back here
   }
 };
+
+// The pool behind AdjBuf, made by the first call on the context and destroyed with it.  It
+// keeps at most ADJ_POOL_KEEP bytes between calls; what a call used above that goes back to
+// the device before it returns.
+constexpr unsigned long long ADJ_POOL_KEEP = 4ULL << 30;
+int adj_pool(dsem_ctx *c) {
+  if (c->adj_pool) return DSEM_OK;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = c->dev;
+  CKA(cudaMemPoolCreate(&c->adj_pool, &props));
+  unsigned long long keep = ADJ_POOL_KEEP;
+  CKA(cudaMemPoolSetAttribute(c->adj_pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  return DSEM_OK;
+}
 
 // Where a group's slices of the adjoint's buffers start (doubles, or elements for e0)
 struct GOff {
@@ -835,8 +863,10 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   if (dJdQ0 && ldx < gmax) return dsem_int::fail(c, DSEM_ERR_INVALID_ARG, "ldx smaller than the number of Gauss points");
   int r = upload_ops_here(c);
   if (r) return r;
+  if ((r = adj_pool(c))) return r;
   Adj A;
   A.c = c;
+  A.b.c = c;
   A.single = c->groups.size() == 1 && c->nnc == 0;
   A.bl = (A.single && c->nbnd > 0) ? &c->blists[0] : nullptr;
   {  // the groups' slices of the buffers
@@ -856,7 +886,7 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
       A.off.push_back(o);
     }
     // p = 7, 8: the volume adjoint's arrays that do not fit shared memory
-    if (scr && cudaMalloc(&A.b.volscr, (size_t)scr * sizeof(double)) != cudaSuccess) {
+    if (scr && A.b.alloc(&A.b.volscr, (size_t)scr * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       return dsem_int::fail(c, DSEM_ERR_NOMEM, "adjoint: not enough device memory for the volume scratch");
     }
@@ -866,31 +896,31 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   A.window = window;
   const size_t nq = c->nq, nf = c->nface, bq = nq * sizeof(double), bf = nf * sizeof(double);
   const int kord = c->kord;
-  for (double **p : {&A.b.lq, &A.b.lg, &A.b.ljq, &A.b.q0}) CKA(cudaMalloc(p, bq));
-  for (double **p : {&A.b.qfr, &A.b.lff, &A.b.lvf, &A.b.lqf, &A.b.lqr}) CKA(cudaMalloc(p, bf));
-  CKA(cudaMalloc(&A.b.lrp, (size_t)c->ngrid * sizeof(double)));
+  for (double **p : {&A.b.lq, &A.b.lg, &A.b.ljq, &A.b.q0}) CKA(A.b.alloc(p, bq));
+  for (double **p : {&A.b.qfr, &A.b.lff, &A.b.lvf, &A.b.lqf, &A.b.lqr}) CKA(A.b.alloc(p, bf));
+  CKA(A.b.alloc(&A.b.lrp, (size_t)c->ngrid * sizeof(double)));
   size_t nbpt = 0;  // boundary points, per list
   for (const BList &bl : c->blists) {
     A.boff.push_back((long long)nbpt);
     nbpt += (size_t)bl.n * bl.G * bl.G;
   }
   if (nbpt) {
-    CKA(cudaMalloc(&A.b.lrb, nbpt * sizeof(double)));
+    CKA(A.b.alloc(&A.b.lrb, nbpt * sizeof(double)));
     CKA(cudaMemsetAsync(A.b.lrb, 0, nbpt * sizeof(double), c->st));
   }
   A.ev = c->shock != 0;
   A.les = c->les != 0;
   A.visc = A.ev || A.les;
   if (A.visc) {
-    CKA(cudaMalloc(&A.b.lmuhg, (nq / 5) * sizeof(double)));
-    CKA(cudaMalloc(&A.b.levb, evb_bytes(A)));
+    CKA(A.b.alloc(&A.b.lmuhg, (nq / 5) * sizeof(double)));
+    CKA(A.b.alloc(&A.b.levb, evb_bytes(A)));
     A.ev_valid0 = grad_flag(A);
     if (A.ev_valid0) {  // the gradients behind the first step's viscosity
-      CKA(cudaMalloc(&A.b.evb0, evb_bytes(A)));
+      CKA(A.b.alloc(&A.b.evb0, evb_bytes(A)));
       if ((r = evb_copy(A, A.b.evb0, true))) return r;
     }
   }
-  CKA(cudaMalloc(&A.b.lr, sizeof(double)));
+  CKA(A.b.alloc(&A.b.lr, sizeof(double)));
   // DSEM_ADJOINT_LEAN=1 takes the paths used when device memory is short: no
   // optional trace or gradient slots and no segment stash (the same results,
   // bit for bit, more work)
@@ -902,24 +932,23 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   if (snapshots > 0 && c->adj_scheme == DSEM_ADJ_SEGMENTS && !lean && A.single && c->nbnd == 0) {
     seg_k = (nsteps + snapshots - 1) / snapshots;
     nseg = (nsteps + seg_k - 1) / seg_k;
-    if (cudaMalloc(&A.b.stages, (size_t)seg_k * kord * bq) != cudaSuccess ||
-        cudaMalloc(&A.b.traces, (size_t)seg_k * kord * bf) != cudaSuccess) {
+    if (A.b.alloc(&A.b.stages, (size_t)seg_k * kord * bq) != cudaSuccess ||
+        A.b.alloc(&A.b.traces, (size_t)seg_k * kord * bf) != cudaSuccess) {
       cudaGetLastError();
-      cudaFree(A.b.stages);
-      cudaFree(A.b.traces);
-      A.b.stages = A.b.traces = nullptr;
+      A.b.release(A.b.stages);
+      A.b.release(A.b.traces);
       seg_k = nseg = 0;
     }
   }
   A.seg_k = seg_k;
   if (!seg_k) {
     const size_t nstage = snapshots == 0 ? (size_t)nsteps * kord : (size_t)kord;
-    if (cudaMalloc(&A.b.stages, nstage * bq) != cudaSuccess) {
+    if (A.b.alloc(&A.b.stages, nstage * bq) != cudaSuccess) {
       cudaGetLastError();
       return dsem_int::fail(c, DSEM_ERR_NOMEM, "adjoint: not enough device memory for the stage states (use snapshots > 0)");
     }
     // raw face traces of every kept stage state (with snapshots: of the step being reversed)
-    if (lean || cudaMalloc(&A.b.traces, nstage * bf) != cudaSuccess) {
+    if (lean || A.b.alloc(&A.b.traces, nstage * bf) != cudaSuccess) {
       cudaGetLastError();  // not enough memory: the reverse sweep recomputes the traces
       A.b.traces = nullptr;
     }
@@ -928,9 +957,9 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   const int nslots = seg_k ? nseg : snapshots;
   for (int s = 0; s < nslots; ++s) {
     double *p = nullptr, *pe = nullptr;
-    if (cudaMalloc(&p, bq) != cudaSuccess || (A.visc && cudaMalloc(&pe, evb_bytes(A)) != cudaSuccess)) {
+    if (A.b.alloc(&p, bq) != cudaSuccess || (A.visc && A.b.alloc(&pe, evb_bytes(A)) != cudaSuccess)) {
       cudaGetLastError();
-      cudaFree(p);
+      A.b.release(p);
       return dsem_int::fail(c, DSEM_ERR_NOMEM, "adjoint: not enough device memory for the snapshots");
     }
     A.b.slots.push_back(p);
@@ -939,7 +968,7 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
       A.b.slot_valid.push_back(0);
     }
   }
-  if (A.visc && A.ckpt) CKA(cudaMalloc(&A.b.evb_prev, evb_bytes(A)));
+  if (A.visc && A.ckpt) CKA(A.b.alloc(&A.b.evb_prev, evb_bytes(A)));
   std::vector<double> tmp(1, dt);
   if ((r = dsem_int::set_dt(c, tmp.data()))) return r;
   cudaEvent_t e0, e1;
@@ -959,17 +988,17 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   // ---- forward sweep
   std::vector<double> s_win;
   const size_t npart = (size_t)c->ngrid * 5;
-  if (window > 0) CKA(cudaMalloc(&A.b.eps_part, (size_t)window * npart * sizeof(double)));
+  if (window > 0) CKA(A.b.alloc(&A.b.eps_part, (size_t)window * npart * sizeof(double)));
   // the gradients saved by each window step's last stage, for the reverse
   // sweep's direct enstrophy term (else recomputed there)
   const size_t nevb = (size_t)3 * c->nq;
   if (oop && !A.visc && window > 0 && !lean &&
-      cudaMalloc(&A.b.evbw, (size_t)window * nevb * sizeof(double)) != cudaSuccess) {
+      A.b.alloc(&A.b.evbw, (size_t)window * nevb * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     A.b.evbw = nullptr;
   }
   if (seg_k && !A.visc && window > 0 &&  // segments: one slot per step of a segment
-      cudaMalloc(&A.b.evbw, (size_t)seg_k * nevb * sizeof(double)) != cudaSuccess) {
+      A.b.alloc(&A.b.evbw, (size_t)seg_k * nevb * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     A.b.evbw = nullptr;
   }

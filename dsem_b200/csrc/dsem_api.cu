@@ -1195,6 +1195,7 @@ void dsem_destroy(dsem_ctx *c) {
   cudaFree(c->flag);
   if (c->e0) cudaEventDestroy(c->e0);
   if (c->e1) cudaEventDestroy(c->e1);
+  if (c->adj_pool) cudaMemPoolDestroy(c->adj_pool);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
