@@ -1128,8 +1128,8 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
   // set the shared-memory attribute of every volume variant outside any capture
   for (auto &g : c->groups)
     for (int mode = 0; mode < 4; ++mode) {
-      VolArgs a{};
-      CK(with_G(g.G, [&](auto gg) { return Launch<decltype(gg)::value>::vol(a, 0, g.diag, mode, c->st); }));
+      VolArgs a{};  // no state: nothing is launched
+      CK(with_G(g.G, [&](auto gg) { return Launch<decltype(gg)::value>::vol(a, g.nel, g.diag, mode, c->st); }));
     }
   return DSEM_OK;
 }

@@ -13,13 +13,14 @@ template <int G> cudaError_t Launch<G>::set_ops(const double *h, int n) {
   return cudaMemcpyToSymbol(c_ops, h, sizeof(double) * OPS_TOTAL);
 }
 
-template <int G, bool DIAG, bool EV, int SAVE> static cudaError_t vol_one(const VolArgs &a, int nel, cudaStream_t s) {
-  using C = VolCfg<G, DIAG, EV, SAVE>;
-  auto kern = k_vol<G, DIAG, EV, SAVE>;
+// general metrics, p = 1, 2
+template <int G, bool EV, int SAVE> static cudaError_t vol_one(const VolArgs &a, int nel, cudaStream_t s) {
+  using C = VolCfg<G, EV>;
+  auto kern = k_vol<G, EV, SAVE>;
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = set_smem_once(kern, C::SMEM, attr);
   if (e != cudaSuccess) return e;
-  if (nel <= 0) return cudaSuccess;
+  if (nel <= 0 || !a.JQ) return cudaSuccess;
   kern<<<nel, C::NT, C::SMEM, s>>>(a);
   return cudaGetLastError();
 }
@@ -31,7 +32,7 @@ template <int G, bool EV, int SAVE> static cudaError_t vol_diag_one(const VolArg
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = set_smem_once(kern, C::SMEM, attr);
   if (e != cudaSuccess) return e;
-  if (nel <= 0) return cudaSuccess;
+  if (nel <= 0 || !a.JQ) return cudaSuccess;
   kern<<<nel, C::NT, C::SMEM, s>>>(a);
   return cudaGetLastError();
 }
@@ -44,9 +45,27 @@ static cudaError_t vol_mma_one(const VolArgs &a, int nel, cudaStream_t s) {
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = set_smem_once(kern, C::SMEM, attr);
   if (e != cudaSuccess) return e;
-  if (nel <= 0) return cudaSuccess;
+  if (nel <= 0 || !a.JQ) return cudaSuccess;
   kern<<<nel, C::NT, C::SMEM, s>>>(a);
   return cudaGetLastError();
+}
+
+// general metrics, p >= 3
+template <int G, bool MU, int SAVE, int V>
+static cudaError_t vol_gen_shape(const VolArgs &a, int nel, cudaStream_t s) {
+  using C = MmaCfg<G, V>;
+  auto kern = k_vol_mma_gen<G, MU, SAVE, V>;
+  static std::atomic<unsigned long long> attr{0};
+  cudaError_t e = set_smem_once(kern, C::SMEM, attr);
+  if (e != cudaSuccess) return e;
+  if (nel <= 0 || !a.JQ) return cudaSuccess;
+  kern<<<nel, C::NT, C::SMEM, s>>>(a);
+  return cudaGetLastError();
+}
+template <int G, bool MU, int SAVE> static cudaError_t vol_gen_one(const VolArgs &a, int nel, cudaStream_t s) {
+  if (G < 8 && nel <= 148 * MmaShape<G, MMA_GEN_WIDE>::MINB)  // (p >= 7: one element per SM anyway)
+    return vol_gen_shape<G, MU, SAVE, (G < 8 ? MMA_GEN_WIDE : MMA_GEN)>(a, nel, s);
+  return vol_gen_shape<G, MU, SAVE, MMA_GEN>(a, nel, s);
 }
 
 // launch shapes of k_vol_mma instantiated for this order (p = 4, 6, 8)
@@ -90,11 +109,20 @@ cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaS
       }
     }
   }
+  if constexpr (G >= VOL_GEN_GMIN) {
+    switch (mode) {
+      case VOL_SAVE: return vol_gen_one<G, false, 1>(a, nel, s);
+      case VOL_EV: return vol_gen_one<G, true, 0>(a, nel, s);
+      case VOL_EV_SAVE: return vol_gen_one<G, true, 2>(a, nel, s);
+      default: return vol_gen_one<G, false, 0>(a, nel, s);
+    }
+  } else {
   switch (mode) {
-    case VOL_SAVE: return vol_one<G, false, false, 1>(a, nel, s);
-    case VOL_EV: return vol_one<G, false, true, 0>(a, nel, s);
-    case VOL_EV_SAVE: return vol_one<G, false, true, 2>(a, nel, s);
-    default: return vol_one<G, false, false, 0>(a, nel, s);
+    case VOL_SAVE: return vol_one<G, false, 1>(a, nel, s);
+    case VOL_EV: return vol_one<G, true, 0>(a, nel, s);
+    case VOL_EV_SAVE: return vol_one<G, true, 2>(a, nel, s);
+    default: return vol_one<G, false, 0>(a, nel, s);
+  }
   }
 }
 

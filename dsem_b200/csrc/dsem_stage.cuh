@@ -30,10 +30,6 @@ __device__ unsigned long long g_phase_cycles[32];
   } while (0)
 #endif
 
-#ifndef DSEM_VOL_THREADS_P8
-#define DSEM_VOL_THREADS_P8 448  // threads per volume CTA for p >= 7 (fastest of 384/448/512 at p = 8)
-#endif
-
 namespace dsem {
 
 // ------------------------------------------------------------------ traces
@@ -801,21 +797,16 @@ struct VolArgs {
   int nel;                      // elements of the launch (set by the launcher)
 };
 
-template <int G, bool DIAG, bool EV, int SAVE> struct VolCfg {
-  static constexpr int L = G + 1, NG = G * G * G, NL = L * G * G;
-  static constexpr int NCH = DIAG ? 11 : 15;          // gradient fields interpolated to each grid
-  static constexpr int NLB = EV ? 6 : 5;              // Lobatto slots (+ EV coefficient)
-  static constexpr size_t MAXS = 232448;              // dynamic shared memory per CTA on sm_100
-  static constexpr size_t bytes(bool pad, bool qsm) {
-    return sizeof(double) *
-           (size_t)(15 * NG + (NLB + NCH) * ((pad ? (L | 1) : L) * G * G) + (qsm ? 5 * NG : 0));
-  }
-  static constexpr bool QSM = bytes(false, true) <= MAXS;  // divergence sum kept in shared memory
-  static constexpr bool PAD = QSM ? bytes(true, true) <= MAXS : bytes(true, false) <= MAXS;
-  static constexpr int LX = PAD ? (L | 1) : L;        // x-grid line stride (odd: no bank conflicts)
-  static constexpr int NLS = LX * G * G;              // stride of one field on a Lobatto grid
-  static constexpr size_t SMEM = bytes(PAD, QSM);
-  static constexpr int NT = G >= 8 ? DSEM_VOL_THREADS_P8 : 256;
+// k_vol: full metrics (rotated, skewed or curved elements) at p = 1, 2, whose lines are too
+// few for the tiles of k_vol_mma_gen.
+template <int G, bool EV> struct VolCfg {
+  static constexpr int L = G + 1, NG = G * G * G;
+  static constexpr int NCH = 15;              // gradient fields interpolated to each grid
+  static constexpr int NLB = EV ? 6 : 5;      // Lobatto slots (+ EV coefficient)
+  static constexpr int LX = L | 1;            // x-grid line stride (odd: no bank conflicts)
+  static constexpr int NLS = LX * G * G;      // stride of one field on a Lobatto grid
+  static constexpr size_t SMEM = sizeof(double) * (size_t)(15 * NG + (NLB + NCH) * NLS + 5 * NG);
+  static constexpr int NT = 256;
 };
 
 // Line (a,b) of direction D on a Lobatto-grid array with x-stride LX.
@@ -884,11 +875,11 @@ __device__ __forceinline__ void deriv_task(int t, const double *LB, int NLS, con
 }
 
 // Pass 2 for one direction: gradients to grid D, fluxes, interior divergence.
-template <int G, bool DIAG, bool EV, int SAVE, int D>
+template <int G, bool EV, int D>
 __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, const double *jac, const double *QF,
                                         const double *gm, const double *muhg, const double *GR, double *LB, double *CH,
                                         double *VF, double *QT, const Phys &P, int tid, int nt, long long &t_ph_) {
-  using C = VolCfg<G, DIAG, EV, SAVE>;
+  using C = VolCfg<G, EV>;
   constexpr int L = G + 1, G2 = G * G, NG = G * G * G, NL = L * G * G;
   constexpr int LX = C::LX, NLS = C::NLS, NCH = C::NCH;
   constexpr int xs = g_stride<G, D>(), ls = lb_stride<G, D>();
@@ -906,26 +897,22 @@ __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, cons
   PHASE_MARK(8 + 4 * D);
   for (int t = tid; t < NCH * G2; t += nt) {  // gradients to grid D (Vis_Fluxes_new.f90:84-109)
     const int jf = t / G2, ln = t - jf * G2, a = ln % G, b = ln / G;
-    const int src = DIAG ? diag_field(D, jf) : jf;
-    contract<G, false, 0, L, 0, G>(GR + src * NG + gbase<G>(D, a, b), xs, CH + jf * NLS + lb_base<G, LX, D>(a, b), ls);
+    contract<G, false, 0, L, 0, G>(GR + jf * NG + gbase<G>(D, a, b), xs, CH + jf * NLS + lb_base<G, LX, D>(a, b), ls);
   }
   __syncthreads();
   PHASE_MARK(9 + 4 * D);
   for (int qi = tid; qi < NL; qi += nt) {  // fluxes on grid D (Vis_Fluxes_new.f90:115-228, fluxesH_newa.f90:276-352)
-    int s, a, b, p, pg;
+    int s, a, b, p;
     if (D == 0) {
       s = qi % L;
       const int r = qi / L;
       a = r % G;
       b = r / G;
       p = s + LX * r;
-      pg = qi;
     } else {
       ldecode<G>(D, qi, s, a, b);
       p = qi;
-      pg = qi;
     }
-    const double gdiag = DIAG ? gm[D * NL + pg] : 0.0;
     double Q[NV], Qx[NV], Qy[NV], Qz[NV], r[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) Q[v] = LB[v * NLS + p];
@@ -933,63 +920,28 @@ __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, cons
     double amu = 1.0;
     if (EV) amu = amu + LB[5 * NLS + p];
     const bool face = (s == 0 || s == L - 1);
-    if (DIAG) {
-      double c[11];
 #pragma unroll
-      for (int jf = 0; jf < 11; ++jf) c[jf] = CH[jf * NLS + p];
-      double fl[NV];
-      if (D == 0) {
-        Qx[0] = c[0]; Qx[1] = c[1]; Qx[2] = c[2]; Qx[3] = c[3]; Qx[4] = c[4];
-        Qy[0] = c[5]; Qy[1] = c[6]; Qy[2] = c[7]; Qy[3] = 0.0; Qy[4] = 0.0;
-        Qz[0] = c[8]; Qz[1] = c[9]; Qz[3] = c[10]; Qz[2] = 0.0; Qz[4] = 0.0;
-        vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, fl);
-      } else if (D == 1) {
-        Qy[0] = c[0]; Qy[1] = c[1]; Qy[2] = c[2]; Qy[3] = c[3]; Qy[4] = c[4];
-        Qx[0] = c[5]; Qx[1] = c[6]; Qx[2] = c[7]; Qx[3] = 0.0; Qx[4] = 0.0;
-        Qz[0] = c[8]; Qz[2] = c[9]; Qz[3] = c[10]; Qz[1] = 0.0; Qz[4] = 0.0;
-        vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, fl);
-      } else {
-        Qz[0] = c[0]; Qz[1] = c[1]; Qz[2] = c[2]; Qz[3] = c[3]; Qz[4] = c[4];
-        Qx[0] = c[5]; Qx[1] = c[6]; Qx[3] = c[7]; Qx[2] = 0.0; Qx[4] = 0.0;
-        Qy[0] = c[8]; Qy[2] = c[9]; Qy[3] = c[10]; Qy[1] = 0.0; Qy[4] = 0.0;
-        vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, fl);
-      }
+    for (int v = 0; v < NV; ++v) {
+      Qx[v] = CH[(v * 3 + 0) * NLS + p];
+      Qy[v] = CH[(v * 3 + 1) * NLS + p];
+      Qz[v] = CH[(v * 3 + 2) * NLS + p];
+    }
+    double f[NV], g[NV], h[NV];
+    vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, f);
+    vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, g);
+    vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, h);
+    const double *g3 = gm + ((long long)D * NL + qi) * 3;
+    const double m0 = g3[0], m1 = g3[1], m2 = g3[2];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) r[v] = gdiag * fl[v];
-      if (face) {
-        const int fc = s == 0 ? face_lo(D) : face_hi(D);
+    for (int v = 0; v < NV; ++v) r[v] = m0 * f[v] + m1 * g[v] + m2 * h[v];
+    if (face) {
+      const int fc = s == 0 ? face_lo(D) : face_hi(D);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) VF[(fc - 1) * 5 * G2 + v * G2 + a + G * b] = r[v];
-      } else {
-        double fi[NV];
-        euler_flux(D, Q, rr, P.gm1, fi);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) CH[v * NLS + p] = gdiag * fi[v] - ddiv(r[v], P.re, P.r_re);
-      }
+      for (int v = 0; v < NV; ++v) VF[(fc - 1) * 5 * G2 + v * G2 + a + G * b] = r[v];
     } else {
+      euler_fluxes3(Q, rr, P.gm1, f, g, h);
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        Qx[v] = CH[(v * 3 + 0) * NLS + p];
-        Qy[v] = CH[(v * 3 + 1) * NLS + p];
-        Qz[v] = CH[(v * 3 + 2) * NLS + p];
-      }
-      double f[NV], g[NV], h[NV];
-      vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, f);
-      vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, g);
-      vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, h);
-      const double *g3 = gm + ((long long)D * NL + pg) * 3;
-      const double m0 = g3[0], m1 = g3[1], m2 = g3[2];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) r[v] = m0 * f[v] + m1 * g[v] + m2 * h[v];
-      if (face) {
-        const int fc = s == 0 ? face_lo(D) : face_hi(D);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) VF[(fc - 1) * 5 * G2 + v * G2 + a + G * b] = r[v];
-      } else {
-        euler_fluxes3(Q, rr, P.gm1, f, g, h);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) CH[v * NLS + p] = (m0 * f[v] + m1 * g[v] + m2 * h[v]) - ddiv(r[v], P.re, P.r_re);
-      }
+      for (int v = 0; v < NV; ++v) CH[v * NLS + p] = (m0 * f[v] + m1 * g[v] + m2 * h[v]) - ddiv(r[v], P.re, P.r_re);
     }
   }
   __syncthreads();
@@ -1013,25 +965,24 @@ __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, cons
   PHASE_MARK(11 + 4 * D);
 }
 
-template <int G, bool DIAG, bool EV, int SAVE>
-__global__ void __launch_bounds__(VolCfg<G, DIAG, EV, SAVE>::NT, 1) k_vol(VolArgs A) {
-  using C = VolCfg<G, DIAG, EV, SAVE>;
-  constexpr int G2 = G * G, NG = C::NG, NL = C::NL, LX = C::LX, NLS = C::NLS;
+template <int G, bool EV, int SAVE>
+__global__ void __launch_bounds__(VolCfg<G, EV>::NT, 1) k_vol(VolArgs A) {
+  using C = VolCfg<G, EV>;
+  constexpr int G2 = G * G, NG = C::NG, NL = C::L * G2, LX = C::LX, NLS = C::NLS;
   extern __shared__ double sm[];
   double *GR = sm;
   double *LB = GR + 15 * NG;
   double *CH = LB + C::NLB * NLS;
-  double *QTS = CH + C::NCH * NLS;  // divergence sum (when it fits)
+  double *QT = CH + C::NCH * NLS;  // divergence sum
   const int k = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const double *JQ = A.JQ + (long long)k * A.sq;
   const double *jac = A.jac + (long long)k * NG;
   const double *QF = A.QF + (long long)k * 30 * G2;
   double *VF = A.VF + (long long)k * 30 * G2;
   double *QTI = A.QTI + (long long)k * 5 * NG;
-  double *QT = C::QSM ? QTS : QTI;
   double *EVB = SAVE ? A.EVB + (long long)k * 15 * NG : nullptr;
-  const double *gg = A.gg + (long long)k * 3 * NG * (DIAG ? 1 : 3);
-  const double *gm = A.gm + (long long)k * 3 * NL * (DIAG ? 1 : 3);
+  const double *gg = A.gg + (long long)k * 9 * NG;
+  const double *gm = A.gm + (long long)k * 9 * NL;
   const double *muhg = EV ? A.muhg + (long long)k * NG : nullptr;
   const double gamma = A.P.gamma;
   Phys P = A.P;
@@ -1057,7 +1008,7 @@ __global__ void __launch_bounds__(VolCfg<G, DIAG, EV, SAVE>::NT, 1) k_vol(VolArg
   PHASE_MARK(1);
   for (int t = tid; t < (NF + 5) * G2; t += nt) {
     if (t < NF * G2)
-      deriv_task<G, LX, DIAG, 0>(t, LB, NLS, gg, GR, EVB, gamma);
+      deriv_task<G, LX, false, 0>(t, LB, NLS, gg, GR, EVB, gamma);
     else
       build_task<G, LX, 1>(t - NF * G2, CH, QF, LB2, NLS);
   }
@@ -1065,25 +1016,23 @@ __global__ void __launch_bounds__(VolCfg<G, DIAG, EV, SAVE>::NT, 1) k_vol(VolArg
   PHASE_MARK(2);
   for (int t = tid; t < (NF + 5) * G2; t += nt) {
     if (t < NF * G2)
-      deriv_task<G, LX, DIAG, 1>(t, LB2, NLS, gg, GR, EVB, gamma);
+      deriv_task<G, LX, false, 1>(t, LB2, NLS, gg, GR, EVB, gamma);
     else
       build_task<G, LX, 2>(t - NF * G2, CH, QF, LB, NLS);
   }
   __syncthreads();
   PHASE_MARK(3);
-  for (int t = tid; t < NF * G2; t += nt) deriv_task<G, LX, DIAG, 2>(t, LB, NLS, gg, GR, EVB, gamma);
+  for (int t = tid; t < NF * G2; t += nt) deriv_task<G, LX, false, 2>(t, LB, NLS, gg, GR, EVB, gamma);
   __syncthreads();
   PHASE_MARK(4);
   if (SAVE) {
     for (int i = tid; i < 12 * NG; i += nt) EVB[i] = GR[i];
   }
   // pass 2: z (reusing the last Lobatto array), y, x
-  vol_dir<G, DIAG, EV, SAVE, 2>(A, JQ, jac, QF, gm, muhg, GR, LB, CH, VF, QT, P, tid, nt, t_ph_);
-  vol_dir<G, DIAG, EV, SAVE, 1>(A, JQ, jac, QF, gm, muhg, GR, LB, CH, VF, QT, P, tid, nt, t_ph_);
-  vol_dir<G, DIAG, EV, SAVE, 0>(A, JQ, jac, QF, gm, muhg, GR, LB, CH, VF, QT, P, tid, nt, t_ph_);
-  if (C::QSM) {
-    for (int i = tid; i < 5 * NG; i += nt) QTI[i] = QTS[i];
-  }
+  vol_dir<G, EV, 2>(A, JQ, jac, QF, gm, muhg, GR, LB, CH, VF, QT, P, tid, nt, t_ph_);
+  vol_dir<G, EV, 1>(A, JQ, jac, QF, gm, muhg, GR, LB, CH, VF, QT, P, tid, nt, t_ph_);
+  vol_dir<G, EV, 0>(A, JQ, jac, QF, gm, muhg, GR, LB, CH, VF, QT, P, tid, nt, t_ph_);
+  for (int i = tid; i < 5 * NG; i += nt) QTI[i] = QT[i];
   PHASE_MARK(20);
 }
 

@@ -60,19 +60,24 @@ __host__ __device__ constexpr int mma_plane(int G) {
 // p = 6, 6 at p = 5 and 10 at p = 4.  Measured, ms of variants 0..4 (22^3 of p = 8, 24^3 of
 // p = 6, 32^3 of p = 4): 1.127 1.156 1.180 1.233 1.307; 0.745 0.762 0.946 0.739 0.854;
 // 0.640 0.708 0.644 0.700 0.671.  Every shape evaluates each value with the same chain.
+// MMA_GEN, MMA_GEN_WIDE: k_vol_mma_gen's shapes (20 shared fields).
 // MMA_WIDE: the shape of variant 0 for launches of at most 148 * MINB elements, which do
 // not fill the GPU: more warps work on one element, and its latency is the launch's.
 // Measured against variant 1's or 0's shape, us: 4^3 elements of p = 8 23.8 (8 warps: 27),
 // p = 6 15.6 (3 warps: 24.7), p = 4 10.4 (2 warps: 16.5); p = 4 at 512 elements, which
 // variant 3 still holds at once, 16.5 with it (2 warps: 19.6).
-constexpr int MMA_WIDE = 5;
+constexpr int MMA_WIDE = 5, MMA_GEN = 6, MMA_GEN_WIDE = 7;
 template <int G, int V> struct MmaShape {
-  static constexpr bool W = V == MMA_WIDE;
-  static constexpr int NW = G >= 8 ? (W ? 16 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 7 : (V == 3 ? 5 : 4)))))
+  static constexpr bool W = V == MMA_WIDE, GEN = V == MMA_GEN, GW = V == MMA_GEN_WIDE;
+  static constexpr int NW = GEN ? (G >= 8 ? 12 : (G == 7 ? 4 : 2))
+                          : GW ? (G >= 7 ? 12 : (G == 6 ? 8 : 4))
+                          : G >= 8 ? (W ? 16 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 7 : (V == 3 ? 5 : 4)))))
                           : G >= 6 ? (W ? (G == 7 ? 12 : 8) : (V == 0 ? 4 : (V == 1 ? 3 : (V == 2 ? 2 : (V == 3 ? 5 : 6)))))
                           : G == 5 ? (W ? 8 : (V <= 2 ? 2 : (V == 3 ? 4 : 3)))
                                    : (W ? 4 : 2);
-  static constexpr int MINB = G >= 8 ? (W ? 1 : 2)
+  static constexpr int MINB = GEN ? (G >= 8 ? 1 : (G == 7 ? 3 : (G == 6 ? 6 : 8)))
+                            : GW ? (G >= 7 ? 1 : (G == 6 ? 1 : 3))
+                            : G >= 8 ? (W ? 1 : 2)
                             : G >= 6 ? (W ? (G == 7 ? 1 : 2) : (V == 3 ? 3 : (V == 4 ? 2 : 4)))
                             : G == 5 ? (W ? 2 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 10 : (V == 3 ? 4 : 5)))))
                                      : (W ? 4 : 8);
@@ -90,7 +95,8 @@ template <int G, int V> struct MmaCfg {
   static constexpr int NLW = (G2 + 31) / 32;            // warps of one line per lane
   static constexpr int NW = MmaShape<G, V>::NW, NT = 32 * NW;
   static constexpr int MINB = MmaShape<G, V>::MINB;
-  static constexpr int NF = 19;  // shared fields: state 5, gradients of fields 0..3 12, energy gradient 2 buffers
+  // shared fields: state 5, gradients of fields 0..3 12, energy gradient 2 buffers (general metrics: 5, 15)
+  static constexpr int NF = V == MMA_GEN || V == MMA_GEN_WIDE ? 20 : 19;
   static constexpr size_t SMEM = sizeof(double) * (size_t)(NF * FS) + 16;
 };
 
@@ -249,6 +255,30 @@ template <int D> __device__ __forceinline__ void mma_add(double *o, double x) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(x) : "memory");
 }
 
+// Interior divergence along D (updatea.f90:100-113) of a tile from its lanes' fluxes, k = s - 1:
+// lane r*4+q gets line r at Gauss points q and 4+q; the ninth Gauss point of G = 9 is a column
+// of its own (q = 0).  qt: the line's first Gauss point.
+template <int G, int V, int D>
+__device__ __forceinline__ void mma_div(const MmaOps<G, V> &O, const double (&f)[2][NV], bool row, int q, double *qt) {
+  using C = MmaCfg<G, V>;
+  constexpr int NG = C::NG, xs = D == 0 ? 1 : (D == 1 ? G : C::G2);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    double e0 = 0.0, e1 = 0.0, g0 = 0.0, g1 = 0.0;
+#pragma unroll
+    for (int j = 0; j < C::NI; ++j) {
+      dmma(e0, e1, f[j][v], O.dm[j]);
+      if (G == 9) dmma(g0, g1, f[j][v], O.d8[j]);
+    }
+    if (row) {
+      double *o = qt + v * NG + q * xs;
+      if (q < G) mma_add<D>(o, e0);
+      if (4 + q < G) mma_add<D>(o + 4 * xs, e1);
+      if (G == 9 && q == 0) mma_add<D>(o + 8 * xs, g0);
+    }
+  }
+}
+
 // One tile of direction D: 8 lines, all their interior Lobatto points.  The
 // state and gradient fields are interpolated, both fluxes evaluated and the
 // interior divergence contracted without leaving the warp's registers.
@@ -299,24 +329,7 @@ __device__ __forceinline__ void mma_tile(int t, const MmaOps<G, V> &O, const Phy
 #pragma unroll
     for (int v = 0; v < NV; ++v) f[i][v] = in ? gd[i] * fi[v] - ddiv(r[v], P.re, P.r_re) : 0.0;
   }
-  // interior divergence along D (updatea.f90:100-113), k = s - 1: lane r*4+q gets line r at
-  // Gauss points q and 4+q; the ninth Gauss point of G = 9 is a column of its own (q = 0)
-  double *qt = QTI + gbase<G>(D, a, b);
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    double e0 = 0.0, e1 = 0.0, g0 = 0.0, g1 = 0.0;
-#pragma unroll
-    for (int j = 0; j < C::NI; ++j) {
-      dmma(e0, e1, f[j][v], O.dm[j]);
-      if (G == 9) dmma(g0, g1, f[j][v], O.d8[j]);
-    }
-    if (row) {
-      double *o = qt + v * NG + q * xs;
-      if (q < G) mma_add<D>(o, e0);
-      if (4 + q < G) mma_add<D>(o + 4 * xs, e1);
-      if (G == 9 && q == 0) mma_add<D>(o + 8 * xs, g0);
-    }
-  }
+  mma_div<G, V, D>(O, f, row, q, QTI + gbase<G>(D, a, b));
 }
 
 // Viscous fluxes at both face points of one line of direction D per lane
@@ -395,8 +408,9 @@ __device__ __forceinline__ void mma_phase(int *next, const MmaOps<G, V> &O, cons
 }
 
 // Temperature gradient along D (EV runs, SAVE == 2): the five Lobatto lines, the
-// temperature on them (RHS.f90:66-83), its derivative scaled by gmetg(D,D).
-template <int G, int V, int D>
+// temperature on them (RHS.f90:66-83), its derivative scaled by gmetg(D,D) (GEN: by
+// gmetg(D,c), added to the three components in the order of the directions).
+template <int G, int V, int D, bool GEN = false>
 __device__ __forceinline__ void mma_tgrad(int ln, const double *sq, const double *QF, const double *gg, double *EVB,
                                           double gamma) {
   constexpr int L = G + 1, G2 = G * G, NG = G * G * G, FS = MmaCfg<G, V>::FS;
@@ -432,7 +446,37 @@ __device__ __forceinline__ void mma_tgrad(int ln, const double *sq, const double
     double acc = Op<G>::D(kk, 0) * T[0];
 #pragma unroll
     for (int s = 1; s < L; ++s) acc = __fma_rn(Op<G>::D(kk, s), T[s], acc);
-    EVB[(12 + D) * NG + p0 + kk * xs] = gg[D * NG + p0 + kk * xs] * acc;
+    const int p = p0 + kk * xs;
+    if (GEN) {  // contributions of direction D to the three components
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double val = gg[p * 9 + D + 3 * c] * acc;
+        EVB[(12 + c) * NG + p] = D == 0 ? val : EVB[(12 + c) * NG + p] + val;
+      }
+    } else {
+      EVB[(12 + D) * NG + p] = gg[D * NG + p] * acc;
+    }
+  }
+}
+
+// Q*jacob (fluxesH_newa.f90:262-272) into the padded state, all of a thread's loads in flight
+// at once.
+template <int G, int NT> __device__ __forceinline__ void mma_load(const double *JQ, const double *jac, double *sq) {
+  constexpr int G2 = G * G, NG = G * G * G, PS = mma_plane(G), NQ = (5 * NG + NT - 1) / NT;
+  const int tid = threadIdx.x;
+  double qv[NQ], jv[NQ];
+#pragma unroll
+  for (int j = 0; j < NQ; ++j) {
+    const int i = tid + j * NT;
+    if (i < 5 * NG) {
+      qv[j] = JQ[i];
+      jv[j] = jac[i % NG];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NQ; ++j) {
+    const int i = tid + j * NT;
+    if (i < 5 * NG) sq[i / G2 * PS + i % G2] = qv[j] * jv[j];
   }
 }
 
@@ -475,24 +519,7 @@ __global__ void __launch_bounds__(MmaCfg<G, V>::NT, MmaCfg<G, V>::MINB) k_vol_mm
 #ifdef DSEM_PHASE_TIMING
   t_ph_ = clock64();
 #endif
-  // Q*jacob (fluxesH_newa.f90:262-272), all of a thread's loads in flight at once
-  {
-    constexpr int NQ = (5 * NG + NT - 1) / NT;
-    double qv[NQ], jv[NQ];
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-      const int i = tid + j * NT;
-      if (i < 5 * NG) {
-        qv[j] = JQ[i];
-        jv[j] = jac[i % NG];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-      const int i = tid + j * NT;
-      if (i < 5 * NG) sq[i / G2 * PS + i % G2] = qv[j] * jv[j];
-    }
-  }
+  mma_load<G, NT>(JQ, jac, sq);
   __syncthreads();
   PHASE_MARK(0);
   MmaOps<G, V> O;
@@ -533,6 +560,248 @@ __global__ void __launch_bounds__(MmaCfg<G, V>::NT, MmaCfg<G, V>::MINB) k_vol_mm
   PHASE_MARK(3);
   mma_phase<G, MU, V, 0>(next + 2, O, P, sq, GR, E0, E1, QF, gg, gm, muhg, nuhg, VF, QTI);
   PHASE_MARK(4);
+}
+
+// ------------------------------------------------------------ general metrics
+// k_vol_mma_gen: the same for elements with full metrics (rotated, skewed or curved), all
+// 15 gradient components kept (k_vol's sums over the directions x, y, z) and all three
+// fluxes formed at every point.  Bound by the FP64 pipe like the diagonal kernel, with about
+// twice its work.  20 shared fields: one element per SM at p >= 7, so 12 warps (168
+// registers) per element.  Measured, ms per volume launch, k_vol -> this: 10^3 curved
+// elements of p = 8 0.415 -> 0.218, p = 7 0.253 -> 0.137, 12^3 of p = 6 0.281 -> 0.171,
+// p = 5 0.169 -> 0.128, 14^3 of p = 4 0.213 -> 0.098, p = 3 0.089 -> 0.048.
+// Contributions of the derivative along D to the Gauss gradients of the five fields on a
+// tile's lines (Gauss_Deriv, SolnDerivsc.f90:36-80): stored for D = 0, added after.
+template <int G, int V, int D>
+__device__ __forceinline__ void mma_gen_grad(int t, const MmaOps<G, V> &O, const double *sq, const double *QF,
+                                             const double *gg, double *GR) {
+  using C = MmaCfg<G, V>;
+  constexpr int L = C::L, G2 = C::G2, FS = C::FS;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int lane = threadIdx.x & 31, q = lane & 3, n = lane >> 2;
+  const bool row = t * 8 + n < G2;
+  int a, b;
+  mma_line<G, D>(row ? t * 8 + n : G2 - 1, a, b);
+  const int pl = mma_base<G, D>(a, b), pq = pl + q * S;
+  const double *m = gg + (gbase<G>(D, a, b) + q * xs) * 9 + D;
+  double mt[3][3];  // [Gauss point q, 4+q, 8][component]
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const bool in = i == 0 ? q < G : (i == 1 ? 4 + q < G : G == 9 && q == 0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) mt[i][c] = in ? __ldg(m + 4 * i * xs * 9 + 3 * c) : 0.0;
+  }
+  const double *flo = QF + (face_lo(D) - 1) * 5 * G2 + a + G * b, *fhi = QF + (face_hi(D) - 1) * 5 * G2 + a + G * b;
+  double y0[NV], y1[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    y0[v] = __ldg(flo + v * G2);
+    y1[v] = __ldg(fhi + v * G2);
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    double c[2];
+    mma_interp<G, V, S>(sq + v * FS + pq, sq + v * FS + pl, O, c[0], c[1]);
+    double w[3] = {O.dlo[0] * y0[v], O.dlo[1] * y0[v], Op<G>::D(G - 1, 0) * y0[v]}, g1 = 0.0;
+#pragma unroll
+    for (int j = 0; j < C::NI; ++j) {
+      dmma(w[0], w[1], c[j], O.dm[j]);
+      if (G == 9) dmma(w[2], g1, c[j], O.d8[j]);
+    }
+    w[0] = __fma_rn(O.dhi[0], y1[v], w[0]);
+    w[1] = __fma_rn(O.dhi[1], y1[v], w[1]);
+    w[2] = __fma_rn(Op<G>::D(G - 1, L - 1), y1[v], w[2]);
+    if (row) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const bool in = i == 0 ? q < G : (i == 1 ? 4 + q < G : G == 9 && q == 0);
+        if (!in) continue;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          double *o = GR + (v * 3 + k) * FS + pq + 4 * i * S;
+          const double val = mt[i][k] * w[i];
+          *o = D == 0 ? val : *o + val;
+        }
+      }
+    }
+  }
+}
+
+// r = m . (viscous fluxes), and with INV also e = m . (Euler fluxes) at one point.
+template <bool INV>
+__device__ __forceinline__ void mma_gen_flux(const double *Q, const double *c, const double *m, double amu,
+                                             const Phys &P, double *r, double *e) {
+  double Qx[NV], Qy[NV], Qz[NV], f[NV], g[NV], h[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    Qx[v] = c[v * 3];
+    Qy[v] = c[v * 3 + 1];
+    Qz[v] = c[v * 3 + 2];
+  }
+  const double rr = 1.0 / Q[0];
+  vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, f);
+  vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, g);
+  vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, h);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) r[v] = m[0] * f[v] + m[1] * g[v] + m[2] * h[v];
+  if (INV) {
+    euler_fluxes3(Q, rr, P.gm1, f, g, h);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) e[v] = m[0] * f[v] + m[1] * g[v] + m[2] * h[v];
+  }
+}
+
+// One tile of direction D (mma_tile with full metrics).
+template <int G, bool MU, int V, int D>
+__device__ __forceinline__ void mma_gen_tile(int t, const MmaOps<G, V> &O, const Phys &P, const double *sq,
+                                             const double *GR, const double *gm, const double *muhg, double *QTI) {
+  using C = MmaCfg<G, V>;
+  constexpr int G2 = C::G2, NG = C::NG, NL = C::NL, FS = C::FS;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int lane = threadIdx.x & 31, q = lane & 3, n = lane >> 2;
+  const bool row = t * 8 + n < G2;
+  int a, b;
+  mma_line<G, D>(row ? t * 8 + n : G2 - 1, a, b);
+  const int pl = mma_base<G, D>(a, b), pq = pl + q * S;
+  const double *g3 = gm + ((long long)D * NL + lbase<G>(D, a, b) + (1 + q) * xs) * 3;
+  double m[2][3], Q[2][NV], c[2][15], mu[2] = {0.0, 0.0}, f[2][NV];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const bool in = i < C::NI && (i == 0 ? 1 : 5) + q <= C::NS;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m[i][k] = in ? __ldg(g3 + i * 12 * xs + k) : 0.0;
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) mma_interp<G, V, S>(sq + v * FS + pq, sq + v * FS + pl, O, Q[0][v], Q[1][v]);
+#pragma unroll
+  for (int j = 0; j < 15; ++j) mma_interp<G, V, S>(GR + j * FS + pq, GR + j * FS + pl, O, c[0][j], c[1][j]);
+  if (MU) {  // EV_Prolong (Prolong_gtol.f90:7-51)
+    const double *x = muhg + gbase<G>(D, a, b);
+    mma_interp<G, V, xs>(x + q * xs, x, O, mu[0], mu[1]);
+  }
+#pragma unroll
+  for (int i = 0; i < C::NI; ++i) {
+    double amu = 1.0, r[NV], e[NV];
+    if (MU) amu = amu + mu[i];
+    mma_gen_flux<true>(Q[i], c[i], m[i], amu, P, r, e);
+    const bool in = (i == 0 ? 1 : 5) + q <= C::NS;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) f[i][v] = in ? e[v] - ddiv(r[v], P.re, P.r_re) : 0.0;
+  }
+  mma_div<G, V, D>(O, f, row, q, QTI + gbase<G>(D, a, b));
+}
+
+// Viscous flux at one face point of a line of direction D per lane (END 0 low, 1 high).
+template <int G, bool MU, int V, int D, int END>
+__device__ __forceinline__ void mma_gen_face(int ln, const Phys &P, const double *QF, const double *GR,
+                                             const double *gm, const double *muhg, double *VF) {
+  using C = MmaCfg<G, V>;
+  constexpr int L = C::L, G2 = C::G2, NL = C::NL, FS = C::FS, s = END ? L - 1 : 0;
+  constexpr int S = mma_stride<G, D>(), xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const int a = ln % G, b = ln / G, pl = mma_base<G, D>(a, b);
+  const int o = ((END ? face_hi(D) : face_lo(D)) - 1) * 5 * G2 + ln;
+  const double *g3 = gm + ((long long)D * NL + lbase<G>(D, a, b) + s * xs) * 3;
+  double Q[NV], m[3], c[15], r[NV];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) m[k] = __ldg(g3 + k);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) Q[v] = __ldg(QF + o + v * G2);
+  auto end = [&](const double *x, int st) {
+    double acc = Op<G>::B(s, 0) * x[0];
+#pragma unroll
+    for (int k = 1; k < G; ++k) acc = __fma_rn(Op<G>::B(s, k), x[k * st], acc);
+    return acc;
+  };
+#pragma unroll
+  for (int j = 0; j < 15; ++j) c[j] = end(GR + j * FS + pl, S);
+  double amu = 1.0;
+  if (MU) amu = amu + end(muhg + gbase<G>(D, a, b), xs);
+  mma_gen_flux<false>(Q, c, m, amu, P, r, nullptr);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) VF[o + v * G2] = r[v];
+}
+
+template <int G, bool MU, int V, int D>
+__device__ __forceinline__ void mma_gen_phase(int *next, const MmaOps<G, V> &O, const Phys &P, const double *sq,
+                                              const double *GR, const double *QF, const double *gm,
+                                              const double *muhg, double *VF, double *QTI) {
+  using C = MmaCfg<G, V>;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = C::NW - 1 - w; i < 2 * C::NLW; i += C::NW) {
+    const int ln = (i >> 1) * 32 + lane;
+    if (ln >= C::G2) continue;
+    if (i & 1)
+      mma_gen_face<G, MU, V, D, 1>(ln, P, QF, GR, gm, muhg, VF);
+    else
+      mma_gen_face<G, MU, V, D, 0>(ln, P, QF, GR, gm, muhg, VF);
+  }
+  __syncwarp();
+  for (;;) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(next, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= C::NTILE) break;
+    mma_gen_tile<G, MU, V, D>(t, O, P, sq, GR, gm, muhg, QTI);
+  }
+}
+
+template <int G, bool MU, int SAVE, int V = MMA_GEN>
+__global__ void __launch_bounds__(MmaCfg<G, V>::NT, MmaCfg<G, V>::MINB) k_vol_mma_gen(VolArgs A) {
+  using C = MmaCfg<G, V>;
+  constexpr int G2 = C::G2, NG = C::NG, NL = C::NL, NT = C::NT, FS = C::FS, PS = C::PS;
+  extern __shared__ double sm[];
+  double *sq = sm;            // [5] state
+  double *GR = sq + 5 * FS;   // [15] Gauss gradients, field v*3 + component
+  int *next = reinterpret_cast<int *>(GR + 15 * FS);
+  const int tid = threadIdx.x, k = blockIdx.x;
+  const double *JQ = A.JQ + (long long)k * A.sq;
+  const double *jac = A.jac + (long long)k * NG;
+  const double *QF = A.QF + (long long)k * 30 * G2;
+  double *VF = A.VF + (long long)k * 30 * G2;
+  const double *gg = A.gg + (long long)k * 9 * NG;
+  const double *gm = A.gm + (long long)k * 9 * NL;
+  const double *muhg = MU ? A.muhg + (long long)k * NG : nullptr;
+  double *EVB = SAVE ? A.EVB + (long long)k * 15 * NG : nullptr;
+  double *QTI = A.QTI + (long long)k * 5 * NG;
+  Phys P = A.P;
+  if (A.rec) {  // per-case Reynolds number
+    const int cs = A.ecase[k];
+    P.re = A.rec[2 * cs];
+    P.r_re = A.rec[2 * cs + 1];
+  }
+  if (tid == 0) {
+    prefetch_l2_bulk(gg, 9 * NG);
+    prefetch_l2_bulk(gm, 9 * NL);
+    prefetch_l2_bulk(QF, 30 * G2);
+    if (MU) prefetch_l2_bulk(muhg, NG);
+  }
+  if (tid < 3) next[tid] = 0;
+  mma_load<G, NT>(JQ, jac, sq);
+  MmaOps<G, V> O;
+  O.load();
+  __syncthreads();
+  // pass 1: Gauss gradients, the directions' contributions added in the order x, y, z
+  for (int t = tid >> 5; t < C::NTILE; t += C::NW) mma_gen_grad<G, V, 0>(t, O, sq, QF, gg, GR);
+  if (SAVE == 2)
+    for (int t = tid; t < G2; t += NT) mma_tgrad<G, V, 0, true>(t, sq, QF, gg, EVB, P.gamma);
+  __syncthreads();
+  for (int t = tid >> 5; t < C::NTILE; t += C::NW) mma_gen_grad<G, V, 1>(t, O, sq, QF, gg, GR);
+  if (SAVE == 2)
+    for (int t = tid; t < G2; t += NT) mma_tgrad<G, V, 1, true>(t, sq, QF, gg, EVB, P.gamma);
+  __syncthreads();
+  for (int t = tid >> 5; t < C::NTILE; t += C::NW) mma_gen_grad<G, V, 2>(t, O, sq, QF, gg, GR);
+  if (SAVE == 2)
+    for (int t = tid; t < G2; t += NT) mma_tgrad<G, V, 2, true>(t, sq, QF, gg, EVB, P.gamma);
+  __syncthreads();
+  if (SAVE) {
+    for (int i = tid; i < 12 * NG; i += NT) EVB[i] = GR[i / G2 * PS + i % G2];
+  }
+  // pass 2: z, y, x
+  mma_gen_phase<G, MU, V, 2>(next + 0, O, P, sq, GR, QF, gm, muhg, VF, QTI);
+  __syncthreads();
+  mma_gen_phase<G, MU, V, 1>(next + 1, O, P, sq, GR, QF, gm, muhg, VF, QTI);
+  __syncthreads();
+  mma_gen_phase<G, MU, V, 0>(next + 2, O, P, sq, GR, QF, gm, muhg, VF, QTI);
 }
 
 }  // namespace dsem
