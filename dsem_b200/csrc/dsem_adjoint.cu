@@ -209,7 +209,7 @@ int face_states(Adj &A, const double *Qs, const double *raw, bool keep_raw) {
   if (r) return r;
   A.launches += (long long)c->mlists.size();
   if (c->nnc > 0) {
-    k_face_nc_inv<<<c->nnc, 128, 0, c->st>>>(c->nc, c->QF, c->FF, c->nc_nh, c->nc_nrm, c->nc_mats, c->P.gamma);
+    k_face_nc_inv<<<c->nnc, NC_THREADS, 0, c->st>>>(c->nc, c->QF, c->FF, c->nc_nh, c->nc_nrm, c->nc_mats, c->P.gamma);
     CKA(cudaGetLastError());
     ++A.launches;
   }

@@ -242,7 +242,7 @@ int enqueue_face_inv(dsem_ctx *c, long long *launches) {
         return Launch<decltype(g)::value>::face_bnd_inv(bl.mb, bl.n, c->QF, c->FF, bl.nh, bl.nrm, bl.qext, BP, st);
       }));
     } else {
-      k_face_nc_inv<<<c->nnc, 128, 0, st>>>(c->nc, c->QF, c->FF, c->nc_nh, c->nc_nrm, c->nc_mats, gamma);
+      k_face_nc_inv<<<c->nnc, NC_THREADS, 0, st>>>(c->nc, c->QF, c->FF, c->nc_nh, c->nc_nrm, c->nc_mats, gamma);
       CK(cudaGetLastError());
     }
     return DSEM_OK;
@@ -306,7 +306,7 @@ int enqueue_face_vis(dsem_ctx *c, long long *launches) {
         return Launch<decltype(g)::value>::face_bnd_vis(bl.mb, bl.n, c->VF, bl.nrm, bl.fvext, st);
       }));
     } else {
-      k_face_nc_vis<<<c->nnc, 128, 0, st>>>(c->nc, c->VF, c->nc_nrm, c->nc_mats);
+      k_face_nc_vis<<<c->nnc, NC_THREADS, 0, st>>>(c->nc, c->VF, c->nc_nrm, c->nc_mats);
       CK(cudaGetLastError());
     }
     return DSEM_OK;
