@@ -127,8 +127,14 @@ cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaS
 }
 
 template <int G> cudaError_t Launch<G>::update(const UpdArgs &a, int nel, cudaStream_t s) {
+  constexpr size_t smem = UPD_SMEM<G>;
+  static std::atomic<unsigned long long> attr[2] = {{0}, {0}};
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        a.fmc ? set_smem_once(k_update<G, true>, smem, attr[1]) : set_smem_once(k_update<G, false>, smem, attr[0]);
+    if (e != cudaSuccess) return e;
+  }
   if (nel <= 0) return cudaSuccess;
-  const size_t smem = sizeof(double) * (30 * G * G + 5 * G * G * G + 2 * G);
   if (a.fmc)
     k_update<G, true><<<nel, 256, smem, s>>>(a);
   else
@@ -174,7 +180,7 @@ cudaError_t Launch<G>::face_inv(const MortarC *mc, int nm, double *QF, double *F
                                 double gamma, cudaStream_t s) {
   if (nm <= 0) return cudaSuccess;
   const long long n = (long long)nm * G * G;
-  k_face_inv<G><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(mc, nm, QF, FF, nh, nrm, gamma);
+  k_face_inv<G><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(mc, nm, QF, FF, nh, nrm, RoeC::of(gamma));
   return cudaGetLastError();
 }
 
@@ -183,7 +189,7 @@ cudaError_t Launch<G>::face_inv_from(const MortarC *mc, int nm, const double *QF
                                      const double *nh, const double *nrm, double gamma, cudaStream_t s) {
   if (nm <= 0) return cudaSuccess;
   const long long n = (long long)nm * G * G;
-  k_face_inv_from<G><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(mc, nm, QFR, QF, FF, nh, nrm, gamma);
+  k_face_inv_from<G><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(mc, nm, QFR, QF, FF, nh, nrm, RoeC::of(gamma));
   return cudaGetLastError();
 }
 

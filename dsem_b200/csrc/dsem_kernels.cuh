@@ -186,21 +186,29 @@ __device__ __forceinline__ void euler_fluxes3(const double *Q, double rr, double
   h[0] = rhow; h[1] = rhou * w; h[2] = rhov * w; h[3] = p + rhow * w; h[4] = w * (rhoe + p);
 }
 
+// Constants of the Roe flux: gamma - 1, gamma / (gamma - 1), (gamma + 1) / 4.  k_face_inv
+// gets them from the host: a division per point and its registers otherwise.
+struct RoeC {
+  double gm1, gg1, gp4;
+  __host__ __device__ static RoeC of(double gamma) {
+    return RoeC{gamma - 1.0, gamma / (gamma - 1.0), (gamma + 1.0) / 4.0};
+  }
+};
+
 // Roe flux with entropy fix (PhysLib.f90:231-320)
-__device__ __forceinline__ void riemann(const double *nh, double ds, const double *Ql, const double *Qr, double gamma,
+__device__ __forceinline__ void riemann(const double *nh, double ds, const double *Ql, const double *Qr, const RoeC &R,
                                         double *flux) {
   double rho = Ql[0], rhou = Ql[1], rhov = Ql[2], rhow = Ql[3], rhoe = Ql[4];
   double rhon = Qr[0], rhoun = Qr[1], rhovn = Qr[2], rhown = Qr[3], rhoen = Qr[4];
   const double rl = 1.0 / rho, rn = 1.0 / rhon;  // divisions by the densities: ddiv (correctly rounded)
   double ul = ddiv(rhou, rho, rl), vl = ddiv(rhov, rho, rl), wl = ddiv(rhow, rho, rl);
-  double pleft = (gamma - 1.0) * (rhoe - ddiv(0.5, rho, rl) * (rhou * rhou + rhov * rhov + rhow * rhow));
+  double pleft = R.gm1 * (rhoe - ddiv(0.5, rho, rl) * (rhou * rhou + rhov * rhov + rhow * rhow));
   double ur = ddiv(rhoun, rhon, rn), vr = ddiv(rhovn, rhon, rn), wr = ddiv(rhown, rhon, rn);
-  double pright = (gamma - 1.0) * (rhoen - ddiv(0.5, rhon, rn) * (rhoun * rhoun + rhovn * rhovn + rhown * rhown));
+  double pright = R.gm1 * (rhoen - ddiv(0.5, rhon, rn) * (rhoun * rhoun + rhovn * rhovn + rhown * rhown));
   double ql = nh[0] * ul + nh[1] * vl + nh[2] * wl;
   double qr = nh[0] * ur + nh[1] * vr + nh[2] * wr;
-  const double gg1 = gamma / (gamma - 1.0);
-  double hl = 0.5 * (ul * ul + vl * vl + wl * wl) + ddiv(gg1 * pleft, rho, rl);
-  double hr = 0.5 * (ur * ur + vr * vr + wr * wr) + ddiv(gg1 * pright, rhon, rn);
+  double hl = 0.5 * (ul * ul + vl * vl + wl * wl) + ddiv(R.gg1 * pleft, rho, rl);
+  double hr = 0.5 * (ur * ur + vr * vr + wr * wr) + ddiv(R.gg1 * pright, rhon, rn);
   double rtd = sqrt(rho * rhon);
   double betal = rho / (rho + rtd);
   double betar = 1.0 - betal;
@@ -208,14 +216,14 @@ __device__ __forceinline__ void riemann(const double *nh, double ds, const doubl
   double vtd = betal * vl + betar * vr;
   double wtd = betal * wl + betar * wr;
   double htd = betal * hl + betar * hr;
-  double atd2 = (gamma - 1.0) * (htd - 0.5 * (utd * utd + vtd * vtd + wtd * wtd));
+  double atd2 = R.gm1 * (htd - 0.5 * (utd * utd + vtd * vtd + wtd * wtd));
   double atd = sqrt(atd2);
   double qtd = utd * nh[0] + vtd * nh[1] + wtd * nh[2];
   if (qtd >= 0.0) {
     double dw1 = 0.5 * ((pright - pleft) / atd2 - (qr - ql) * rtd / atd);
     double sp1 = qtd - atd;
     double sp1m = sp1 <= 0.0 ? sp1 : 0.0;
-    double hd1m = ((gamma + 1.0) / 4.0 * atd / rtd) * dw1;
+    double hd1m = (R.gp4 * atd / rtd) * dw1;
     double e1 = -fabs(sp1) - hd1m;
     double eta1 = e1 >= 0.0 ? e1 : 0.0;
     double udw1 = dw1 * (sp1m - 0.5 * eta1);
@@ -229,7 +237,7 @@ __device__ __forceinline__ void riemann(const double *nh, double ds, const doubl
     double dw4 = 0.5 * ((pright - pleft) / atd2 + (qr - ql) * rtd / atd);
     double sp4 = qtd + atd;
     double sp4p = sp4 >= 0.0 ? sp4 : 0.0;
-    double hd4 = ((gamma + 1.0) / 4.0 * atd / rtd) * dw4;
+    double hd4 = (R.gp4 * atd / rtd) * dw4;
     double e4 = -fabs(sp4) + hd4;
     double eta4 = e4 >= 0.0 ? e4 : 0.0;
     double udw4 = dw4 * (sp4p + 0.5 * eta4);
@@ -240,6 +248,10 @@ __device__ __forceinline__ void riemann(const double *nh, double ds, const doubl
     flux[3] = ds * (rqr * wr + pright * nh[2] - udw4 * (wtd + atd * nh[2]));
     flux[4] = ds * (rqr * hr - udw4 * (htd + qtd * atd));
   }
+}
+__device__ __forceinline__ void riemann(const double *nh, double ds, const double *Ql, const double *Qr, double gamma,
+                                        double *flux) {
+  riemann(nh, ds, Ql, Qr, RoeC::of(gamma), flux);
 }
 
 // Viscous fluxes (PhysLib.f90:419-583).  GX/GY/GZ hold the gradient

@@ -33,37 +33,33 @@ __device__ unsigned long long g_phase_cycles[32];
 namespace dsem {
 
 // ------------------------------------------------------------------ traces
-template <int G, int HI> __device__ __forceinline__ double trace_of(const double *x, int xs) {
-  constexpr int n = HI ? G : 0;  // Lobatto end point (L-1 = G)
-  double acc = Op<G>::B(n, 0) * x[0];
+// Both face traces of one line of direction D of field v in q (Gauss layout, smem): the two
+// chains share the line's loads.
+template <int G, int D> __device__ __forceinline__ void trace_line(const double *q, int v, int ln, double *QF) {
+  constexpr int G2 = G * G, NG = G * G * G, xs = D == 0 ? 1 : (D == 1 ? G : G2);
+  const double *x = q + v * NG + gbase<G>(D, ln % G, ln / G);
+  double lo = Op<G>::B(0, 0) * x[0], hi = Op<G>::B(G, 0) * x[0];
 #pragma unroll
-  for (int j = 1; j < G; ++j) acc = __fma_rn(Op<G>::B(n, j), x[j * xs], acc);
-  return acc;
+  for (int j = 1; j < G; ++j) {
+    const double xv = x[j * xs];
+    lo = __fma_rn(Op<G>::B(0, j), xv, lo);
+    hi = __fma_rn(Op<G>::B(G, j), xv, hi);
+  }
+  QF[((face_lo(D) - 1) * 5 + v) * G2 + ln] = lo;
+  QF[((face_hi(D) - 1) * 5 + v) * G2 + ln] = hi;
 }
 
 // all six face traces of the 5 fields in q (Gauss layout, smem) -> QF slots
 template <int G> __device__ __forceinline__ void write_traces(const double *q, double *QF, int tid, int nt) {
-  constexpr int G2 = G * G, NG = G * G * G;
-  for (int t = tid; t < 30 * G2; t += nt) {
-    const int f = t / (5 * G2);  // 0..5 -> faces 1..6
-    const int r = t - f * 5 * G2;
-    const int v = r / G2, ln = r - v * G2;
-    const int a = ln % G, b = ln / G;
-    const int face = f + 1;
-    const int d = (face == 4 || face == 6) ? 0 : ((face == 1 || face == 2) ? 1 : 2);
-    const double *x = q + v * NG;
-    double val;
-    if (d == 0) {
-      x += gbase<G>(0, a, b);
-      val = (face == 4) ? trace_of<G, 1>(x, 1) : trace_of<G, 0>(x, 1);
-    } else if (d == 1) {
-      x += gbase<G>(1, a, b);
-      val = (face == 2) ? trace_of<G, 1>(x, G) : trace_of<G, 0>(x, G);
-    } else {
-      x += gbase<G>(2, a, b);
-      val = (face == 5) ? trace_of<G, 1>(x, G2) : trace_of<G, 0>(x, G2);
-    }
-    QF[t] = val;
+  constexpr int G2 = G * G;
+  for (int t = tid; t < 15 * G2; t += nt) {
+    const int dv = t / G2, ln = t - dv * G2, d = dv / 5, v = dv - d * 5;
+    if (d == 0)
+      trace_line<G, 0>(q, v, ln, QF);
+    else if (d == 1)
+      trace_line<G, 1>(q, v, ln, QF);
+    else
+      trace_line<G, 2>(q, v, ln, QF);
   }
 }
 
@@ -113,7 +109,7 @@ template <int G> __device__ __forceinline__ void slave_index(int orient, int i, 
 template <int G>
 __device__ __forceinline__ void face_inv_point(const MortarC &M, int pt, const double *QFin, double *QF,
                                                double *__restrict__ FF, const double *__restrict__ nh,
-                                               const double *__restrict__ nrm, double gamma) {
+                                               const double *__restrict__ nrm, const RoeC &R) {
   constexpr int G2 = G * G;
   const int i = pt % G, j = pt / G;
   int si, sj;
@@ -128,7 +124,7 @@ __device__ __forceinline__ void face_inv_point(const MortarC &M, int pt, const d
   const long long gp = (long long)M.geo * G2 + pt;
   const double n3[3] = {nh[gp * 3], nh[gp * 3 + 1], nh[gp * 3 + 2]};
   const bool low = (M.flags >> 5) & 1;
-  riemann(n3, nrm[gp], low ? Q2 : Q1, low ? Q1 : Q2, gamma, f);
+  riemann(n3, nrm[gp], low ? Q2 : Q1, low ? Q1 : Q2, R, f);
   const double sgn = ((M.flags >> 3) & 1) ? -1.0 : 1.0;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -143,12 +139,12 @@ __device__ __forceinline__ void face_inv_point(const MortarC &M, int pt, const d
 template <int G>
 __global__ void __launch_bounds__(128) k_face_inv(const MortarC *__restrict__ mc, int nm, double *QF,
                                                    double *__restrict__ FF, const double *__restrict__ nh,
-                                                   const double *__restrict__ nrm, double gamma) {
+                                                   const double *__restrict__ nrm, RoeC R) {
   constexpr int G2 = G * G;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)nm * G2) return;
   const int m = (int)(t / G2), pt = (int)(t - (long long)m * G2);
-  face_inv_point<G>(mc[m], pt, QF, QF, FF, nh, nrm, gamma);
+  face_inv_point<G>(mc[m], pt, QF, QF, FF, nh, nrm, R);
 }
 
 // The same with the raw traces kept elsewhere (QFR, left unchanged).
@@ -156,12 +152,12 @@ template <int G>
 __global__ void __launch_bounds__(128) k_face_inv_from(const MortarC *__restrict__ mc, int nm,
                                                         const double *__restrict__ QFR, double *__restrict__ QF,
                                                         double *__restrict__ FF, const double *__restrict__ nh,
-                                                        const double *__restrict__ nrm, double gamma) {
+                                                        const double *__restrict__ nrm, RoeC R) {
   constexpr int G2 = G * G;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)nm * G2) return;
   const int m = (int)(t / G2), pt = (int)(t - (long long)m * G2);
-  face_inv_point<G>(mc[m], pt, QFR, QF, FF, nh, nrm, gamma);
+  face_inv_point<G>(mc[m], pt, QFR, QF, FF, nh, nrm, R);
 }
 
 template <int G>
@@ -1091,8 +1087,7 @@ struct UpdArgs {
 // at its slave image: the value that the face on side `side` (0 master, 1 slave) receives,
 // with k_face_vis's operations in k_face_vis's order.
 __device__ __forceinline__ double vis_avg_point(const MortarC &M, int side, double vm, double vs, double nm_m,
-                                                double nm_s) {
-  const double rm = 1.0 / nm_m, rs = 1.0 / nm_s;
+                                                double nm_s, double rm, double rs) {
   const bool neg_n = (M.flags >> 4) & 1, neg_s = (M.flags >> 3) & 1;
   const double fv1 = ddiv(vm, nm_m, rm);
   const double fv2 = ddiv(vs, nm_s, rs);
@@ -1101,14 +1096,43 @@ __device__ __forceinline__ double vis_avg_point(const MortarC &M, int side, doub
   return side ? (neg_s ? -qb : qb) : qb;
 }
 
+// What bounds it: HBM, once the index arithmetic, divisions and shared-memory reads are out of
+// the way.  A thread per (face, point) takes the five fields of the BR1 average together, so
+// indices, norms and the two reciprocals are formed once instead of five times; a thread per
+// (direction, field, line) writes both face traces from one read of the line.  Update at 22^3
+// elements of p = 8: 0.422 -> 0.315 ms; 20^3
+// p = 7 0.225 -> 0.168, 24^3 p = 6 0.324 -> 0.239, p = 5 0.227 -> 0.161.  Up to p = 4 a block is
+// short and its dependent load phases (mortar table, faces, state) set the time: there the
+// state's arrays are requested first, by cp.async into shared memory, and arrive during the
+// face phase (32^3 p = 4: 0.386 -> 0.315 -> 0.289 ms with it; at p = 6 and 8 the larger blocks
+// lose more occupancy than they gain, 0.239 -> 0.272 at p = 6).
+template <int G> constexpr bool UPD_STAGED = G <= 5;
+template <int G> constexpr size_t UPD_SMEM = sizeof(double) * (30 * G * G + 5 * G * G * G + 2 * G + (UPD_STAGED<G> ? 11 * G * G * G : 0));
+
+__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+
 template <int G, bool FV = false> __global__ void __launch_bounds__(256) k_update(UpdArgs A) {
   constexpr int L = G + 1, G2 = G * G, NG = G * G * G;
+  constexpr bool STG = UPD_STAGED<G>;
   extern __shared__ double sm[];
   double *FB = sm;            // 30*G2 face fluxes
   double *QN = FB + 30 * G2;  // 5*NG updated physical Q
   double *Dlo = QN + 5 * NG;  // first and last columns of dmx
   double *Dhi = Dlo + G;
+  double *SQ = Dhi + G, *SG = SQ + 5 * NG, *SJ = SG + 5 * NG;  // STG: QTI, gQ, jac (JQ in QN's place)
   const int k = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  if constexpr (STG) {
+    const double *qti = A.QTI + (long long)k * 5 * NG, *jq = A.JQ + (long long)k * A.sq, *gq = A.gQ + (long long)k * A.sq;
+    for (int i = tid; i < 5 * NG; i += nt) {
+      cp_async8(SQ + i, qti + i);
+      cp_async8(QN + i, jq + i);
+      if (A.update && !A.first) cp_async8(SG + i, gq + i);
+    }
+    for (int i = tid; i < NG; i += nt) cp_async8(SJ + i, A.jac + (long long)k * NG + i);
+  }
   const double *FF = A.FF + (long long)k * 30 * G2;
   const double *VF = A.VF + (long long)k * 30 * G2;
   double re = A.re, rre = A.r_re, cdt = A.cdt;
@@ -1139,41 +1163,34 @@ template <int G, bool FV = false> __global__ void __launch_bounds__(256) k_updat
       }
     }
   } else {
-    // the element's six mortars, then per item (face f, field v, mortar point pt) the
-    // BR1 average of k_face_vis into this face's slot (pt on a master face, the point
-    // sp that the orientation maps pt to on a slave face); four items per thread in flight
+    // the element's six mortars, then per item (face f, mortar point pt) the BR1 averages of
+    // k_face_vis into this face's slots (pt on a master face, the point sp that the
+    // orientation maps pt to on a slave face); the five fields share the indices, the norms
+    // and their reciprocals, and have 15 loads in flight
     __shared__ MortarC FM[6];
     if (tid < 6) FM[tid] = A.fmc[6LL * k + tid];
     __syncthreads();
-    constexpr int UF = 4;
-    for (int i0 = tid; i0 < 30 * G2; i0 += UF * nt) {
-      double ff[UF], vm[UF], vs[UF], nm[UF], ns[UF];
-      int own[UF];
+    for (int i = tid; i < 6 * G2; i += nt) {
+      const int f = i / G2, pt = i - f * G2;
+      const MortarC &M = FM[f];
+      int si, sj;
+      slave_index<G>(M.flags & 7, pt % G, pt / G, si, sj);
+      const int sp = si + G * sj, side = (M.flags >> 8) & 1, own = f * 5 * G2 + (side ? sp : pt);
+      const double *vmp = A.VFr + M.ms + pt, *vsp = A.VFr + M.ss + sp;
+      double ff[NV], vm[NV], vs[NV];
 #pragma unroll
-      for (int u = 0; u < UF; ++u) {
-        const int i = i0 + u * nt;
-        own[u] = -1;
-        if (i < 30 * G2) {
-          const int f = i / (5 * G2), r = i - f * 5 * G2, v = r / G2, pt = r - v * G2;
-          const MortarC &M = FM[f];
-          int si, sj;
-          slave_index<G>(M.flags & 7, pt % G, pt / G, si, sj);
-          const int sp = si + G * sj;
-          own[u] = f * 5 * G2 + v * G2 + (((M.flags >> 8) & 1) ? sp : pt);
-          const long long g0 = (long long)M.geo * G2;
-          ff[u] = FF[own[u]];
-          vm[u] = A.VFr[M.ms + v * G2 + pt];
-          vs[u] = A.VFr[M.ss + v * G2 + sp];
-          nm[u] = A.vnrm[g0 + pt];
-          ns[u] = A.vnrm[g0 + sp];
-        }
+      for (int v = 0; v < NV; ++v) {
+        ff[v] = FF[own + v * G2];
+        vm[v] = vmp[v * G2];
+        vs[v] = vsp[v * G2];
       }
+      const double *nrm = A.vnrm + (long long)M.geo * G2;
+      const double nm_m = nrm[pt], nm_s = nrm[sp];
+      const double rm = 1.0 / nm_m, rs = 1.0 / nm_s;
 #pragma unroll
-      for (int u = 0; u < UF; ++u) {
-        if (own[u] < 0) continue;
-        const MortarC &M = FM[own[u] / (5 * G2)];
-        const double vf = vis_avg_point(M, (M.flags >> 8) & 1, vm[u], vs[u], nm[u], ns[u]);
-        FB[own[u]] = ff[u] - ddiv(vf, re, rre);
+      for (int v = 0; v < NV; ++v) {
+        const double vf = vis_avg_point(M, side, vm[v], vs[v], nm_m, nm_s, rm, rs);
+        FB[own + v * G2] = ff[v] - ddiv(vf, re, rre);
       }
     }
   }
@@ -1181,12 +1198,14 @@ template <int G, bool FV = false> __global__ void __launch_bounds__(256) k_updat
     Dlo[i] = Op<G>::D(i, 0);
     Dhi[i] = Op<G>::D(i, L - 1);
   }
+  if constexpr (STG) asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   double *JQ = A.JQ + (long long)k * A.sq;
   double *JQw = A.JQo ? A.JQo + (long long)k * A.sq : JQ;  // where the updated state goes
   double *gQ = A.gQ + (long long)k * A.sq;
   const double *QTI = A.QTI + (long long)k * 5 * NG;
   const double *jac = A.jac + (long long)k * NG;
+  const bool use_g = A.update && !A.first;
   bool bad = false;
   constexpr int U = 2;  // items per thread with their loads in flight together
   for (int i0 = tid; i0 < 5 * NG; i0 += U * nt) {
@@ -1195,10 +1214,10 @@ template <int G, bool FV = false> __global__ void __launch_bounds__(256) k_updat
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * nt;
       if (i < 5 * NG) {
-        qti[u] = QTI[i];
-        jq[u] = JQ[i];
-        gq[u] = (A.update && !A.first) ? gQ[i] : 0.0;
-        jc[u] = jac[i % NG];
+        qti[u] = STG ? SQ[i] : QTI[i];
+        jq[u] = STG ? QN[i] : JQ[i];
+        gq[u] = use_g ? (STG ? SG[i] : gQ[i]) : 0.0;
+        jc[u] = STG ? SJ[i % NG] : jac[i % NG];
       }
     }
 #pragma unroll
