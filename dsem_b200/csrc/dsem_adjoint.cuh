@@ -1,6 +1,6 @@
 // dsem_adjoint.cuh -- discrete adjoint of one right-hand side evaluation.
 //
-// Forward (one stage, dsem_stage.cuh / dsem_vol_diag.cuh):
+// Forward (one stage, dsem_stage.cuh / dsem_vol_mma.cuh):
 //   q = JQ jacob -> face traces QFR -> mortars: Roe flux FF, averaged state QF
 //   -> volume: Lobatto arrays, Gauss gradients, fluxes, interior divergence QTI,
 //      viscous face flux VF -> BR1 average of VF -> Qt = -(QTI + face terms(FF - VF/Re)).
