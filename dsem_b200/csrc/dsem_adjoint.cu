@@ -62,41 +62,77 @@ struct AdjBuf {
   double *evb_prev = nullptr;
   double *lrb = nullptr;  // boundary faces: per boundary point, dJ/d(1/Re) of the external viscous flux
   double *volscr = nullptr;  // p = 7, 8: the volume adjoint's per element scratch (VolAdjCfg::SCR)
-  // Device memory from the context's pool, in stream order: cudaMalloc and cudaFree of these
-  // buffers took 11 ms and more of a 44 ms call (8^3 elements of p = 6, 30 steps) and up to
-  // 170 ms when the driver unmapped them; from the pool a repeated call finds them mapped.
+  // Device memory: one block for all buffers of the call, or, when that cannot be had, a
+  // cudaMalloc per buffer, so that the optional ones can fail one by one.  Measured for 18
+  // buffers of 2.25 GB together (8^3 elements of p = 6, 30 steps, every stage kept): 18 x
+  // (cudaMalloc + cudaFree) 13.8 ms and now and then 290; one pair 2.5.  A stream-ordered pool
+  // maps and unmaps by the byte: 28 ms for its first use and its end, 0.04 between them; at
+  // 0.3 GB 3.9 against 11 and 0.9.  So a block of at most ADJ_POOL_KEEP comes from the
+  // context's pool, which keeps it for the next call (the driver takes it back when another
+  // allocation needs the memory), and a larger one is mapped and freed by the call.
   dsem_ctx *c = nullptr;
+  char *block = nullptr;
+  size_t size = 0, used = 0;
+  bool pooled = false;
+  std::vector<double *> own;  // buffers with a cudaMalloc of their own
+  static size_t padded(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+  void reserve(size_t bytes);
   cudaError_t alloc(double **p, size_t bytes) {
-    return cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, c->adj_pool, c->st);
+    if (block && padded(bytes) <= size - used) {
+      *p = reinterpret_cast<double *>(block + used);
+      used += padded(bytes);
+      return cudaSuccess;
+    }
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) own.push_back(*p);
+    return e;
   }
-  void release(double *&p) {
-    if (p) cudaFreeAsync(p, c->st);
+  void release(double *&p) {  // (a part of the block is given back with it)
+    const auto it = std::find(own.begin(), own.end(), p);
+    if (p && it != own.end()) {
+      cudaFree(p);
+      own.erase(it);
+    }
     p = nullptr;
   }
   ~AdjBuf() {
-    for (double **p : {&lq, &lg, &ljq, &qfr, &lff, &lvf, &lqf, &lqr, &lrp, &lr, &q0, &stages, &traces, &lmuhg, &levb,
-                       &evb0, &eps_part, &evbw, &evb_prev, &lrb, &volscr})
-      release(*p);
-    for (double *&p : slots) release(p);
-    for (double *&p : slot_evb) release(p);
-    if (c) cudaStreamSynchronize(c->st);  // what the pool does not keep is given back here
+    for (double *p : own) cudaFree(p);
+    if (pooled) {
+      cudaFreeAsync(block, c->st);
+      cudaStreamSynchronize(c->st);  // what the pool does not keep is given back here
+    } else {
+      cudaFree(block);
+    }
   }
 };
 
-// The pool behind AdjBuf, made by the first call on the context and destroyed with it.  It
-// keeps at most ADJ_POOL_KEEP bytes between calls; what a call used above that goes back to
-// the device before it returns.
-constexpr unsigned long long ADJ_POOL_KEEP = 4ULL << 30;
-int adj_pool(dsem_ctx *c) {
-  if (c->adj_pool) return DSEM_OK;
+// The pool of the smaller blocks, made by the first call that needs it and destroyed with the
+// context.  It keeps at most ADJ_POOL_KEEP bytes between calls: 256 MiB, below which its first
+// use and its end together still take less than the separate allocations did.
+constexpr size_t ADJ_POOL_KEEP = (size_t)256 << 20;
+bool adj_pool(dsem_ctx *c) {
+  if (c->adj_pool) return true;
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = c->dev;
-  CKA(cudaMemPoolCreate(&c->adj_pool, &props));
   unsigned long long keep = ADJ_POOL_KEEP;
-  CKA(cudaMemPoolSetAttribute(c->adj_pool, cudaMemPoolAttrReleaseThreshold, &keep));
-  return DSEM_OK;
+  if (cudaMemPoolCreate(&c->adj_pool, &props) != cudaSuccess) {
+    c->adj_pool = nullptr;
+    return false;
+  }
+  return cudaMemPoolSetAttribute(c->adj_pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
+}
+
+void AdjBuf::reserve(size_t bytes) {
+  void *p = nullptr;
+  if (bytes <= ADJ_POOL_KEEP)
+    pooled = adj_pool(c) && cudaMallocFromPoolAsync(&p, bytes, c->adj_pool, c->st) == cudaSuccess;
+  if (pooled || cudaMalloc(&p, bytes) == cudaSuccess) {
+    block = static_cast<char *>(p);
+    size = bytes;
+  }
+  cudaGetLastError();
 }
 
 // Where a group's slices of the adjoint's buffers start (doubles, or elements for e0)
@@ -863,64 +899,39 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   if (dJdQ0 && ldx < gmax) return dsem_int::fail(c, DSEM_ERR_INVALID_ARG, "ldx smaller than the number of Gauss points");
   int r = upload_ops_here(c);
   if (r) return r;
-  if ((r = adj_pool(c))) return r;
   Adj A;
   A.c = c;
   A.b.c = c;
   A.single = c->groups.size() == 1 && c->nnc == 0;
   A.bl = (A.single && c->nbnd > 0) ? &c->blists[0] : nullptr;
-  {  // the groups' slices of the buffers
-    long long scr = 0;
-    for (const Group &g : c->groups) {
-      GOff o;
-      o.q0 = g.q0;
-      o.f0 = g.f0;
-      o.e0 = g.e0;
-      o.gq = g.q0 / 5;
-      o.ev = 3 * g.q0;
-      o.scr = scr;
-      with_G(g.G, [&](auto gc) -> cudaError_t {
-        scr += (long long)VolAdjCfg<decltype(gc)::value>::SCR * g.nel;
-        return cudaSuccess;
-      });
-      A.off.push_back(o);
-    }
-    // p = 7, 8: the volume adjoint's arrays that do not fit shared memory
-    if (scr && A.b.alloc(&A.b.volscr, (size_t)scr * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      return dsem_int::fail(c, DSEM_ERR_NOMEM, "adjoint: not enough device memory for the volume scratch");
-    }
-  }
-  A.dt = dt;
-  A.nsteps = nsteps;
-  A.window = window;
+  A.ev = c->shock != 0;
+  A.les = c->les != 0;
+  A.visc = A.ev || A.les;
+  A.ckpt = snapshots > 0;
+  A.ev_valid0 = A.visc && grad_flag(A);
   const size_t nq = c->nq, nf = c->nface, bq = nq * sizeof(double), bf = nf * sizeof(double);
+  const size_t npart = (size_t)c->ngrid * 5, nevb = (size_t)3 * c->nq;
   const int kord = c->kord;
-  for (double **p : {&A.b.lq, &A.b.lg, &A.b.ljq, &A.b.q0}) CKA(A.b.alloc(p, bq));
-  for (double **p : {&A.b.qfr, &A.b.lff, &A.b.lvf, &A.b.lqf, &A.b.lqr}) CKA(A.b.alloc(p, bf));
-  CKA(A.b.alloc(&A.b.lrp, (size_t)c->ngrid * sizeof(double)));
+  long long scr = 0;
+  for (const Group &g : c->groups) {  // the groups' slices of the buffers
+    GOff o;
+    o.q0 = g.q0;
+    o.f0 = g.f0;
+    o.e0 = g.e0;
+    o.gq = g.q0 / 5;
+    o.ev = 3 * g.q0;
+    o.scr = scr;
+    with_G(g.G, [&](auto gc) -> cudaError_t {
+      scr += (long long)VolAdjCfg<decltype(gc)::value>::SCR * g.nel;
+      return cudaSuccess;
+    });
+    A.off.push_back(o);
+  }
   size_t nbpt = 0;  // boundary points, per list
   for (const BList &bl : c->blists) {
     A.boff.push_back((long long)nbpt);
     nbpt += (size_t)bl.n * bl.G * bl.G;
   }
-  if (nbpt) {
-    CKA(A.b.alloc(&A.b.lrb, nbpt * sizeof(double)));
-    CKA(cudaMemsetAsync(A.b.lrb, 0, nbpt * sizeof(double), c->st));
-  }
-  A.ev = c->shock != 0;
-  A.les = c->les != 0;
-  A.visc = A.ev || A.les;
-  if (A.visc) {
-    CKA(A.b.alloc(&A.b.lmuhg, (nq / 5) * sizeof(double)));
-    CKA(A.b.alloc(&A.b.levb, evb_bytes(A)));
-    A.ev_valid0 = grad_flag(A);
-    if (A.ev_valid0) {  // the gradients behind the first step's viscosity
-      CKA(A.b.alloc(&A.b.evb0, evb_bytes(A)));
-      if ((r = evb_copy(A, A.b.evb0, true))) return r;
-    }
-  }
-  CKA(A.b.alloc(&A.b.lr, sizeof(double)));
   // DSEM_ADJOINT_LEAN=1 takes the paths used when device memory is short: no
   // optional trace or gradient slots and no segment stash (the same results,
   // bit for bit, more work)
@@ -932,6 +943,55 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   if (snapshots > 0 && c->adj_scheme == DSEM_ADJ_SEGMENTS && !lean && A.single && c->nbnd == 0) {
     seg_k = (nsteps + snapshots - 1) / snapshots;
     nseg = (nsteps + seg_k - 1) / seg_k;
+  }
+  {  // all buffers below, the optional ones included, in one block
+    const size_t kept = (size_t)kord * (seg_k ? seg_k : snapshots == 0 ? nsteps : 1);  // stage states
+    const int slots = seg_k ? nseg : snapshots;
+    size_t n = 0;
+    auto add = [&](size_t count, size_t bytes) { n += count * AdjBuf::padded(bytes); };
+    add(1, (size_t)scr * sizeof(double));
+    add(4, bq);
+    add(5, bf);
+    add(1, (size_t)c->ngrid * sizeof(double));
+    add(1, nbpt * sizeof(double));
+    add(1, sizeof(double));
+    add(1, kept * bq);
+    if (!lean) add(1, kept * bf);
+    add(slots, bq);
+    if (A.visc) {
+      add(1, (nq / 5) * sizeof(double));
+      add(1 + (A.ev_valid0 ? 1 : 0) + slots + (A.ckpt ? 1 : 0), evb_bytes(A));
+    }
+    add(1, (size_t)window * npart * sizeof(double));
+    if (!A.visc && !lean && (seg_k || (snapshots == 0 && A.single && c->nbnd == 0)))
+      add(1, (size_t)(seg_k && window > 0 ? seg_k : window) * nevb * sizeof(double));
+    A.b.reserve(n);
+  }
+  // p = 7, 8: the volume adjoint's arrays that do not fit shared memory
+  if (scr && A.b.alloc(&A.b.volscr, (size_t)scr * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    return dsem_int::fail(c, DSEM_ERR_NOMEM, "adjoint: not enough device memory for the volume scratch");
+  }
+  A.dt = dt;
+  A.nsteps = nsteps;
+  A.window = window;
+  for (double **p : {&A.b.lq, &A.b.lg, &A.b.ljq, &A.b.q0}) CKA(A.b.alloc(p, bq));
+  for (double **p : {&A.b.qfr, &A.b.lff, &A.b.lvf, &A.b.lqf, &A.b.lqr}) CKA(A.b.alloc(p, bf));
+  CKA(A.b.alloc(&A.b.lrp, (size_t)c->ngrid * sizeof(double)));
+  if (nbpt) {
+    CKA(A.b.alloc(&A.b.lrb, nbpt * sizeof(double)));
+    CKA(cudaMemsetAsync(A.b.lrb, 0, nbpt * sizeof(double), c->st));
+  }
+  if (A.visc) {
+    CKA(A.b.alloc(&A.b.lmuhg, (nq / 5) * sizeof(double)));
+    CKA(A.b.alloc(&A.b.levb, evb_bytes(A)));
+    if (A.ev_valid0) {  // the gradients behind the first step's viscosity
+      CKA(A.b.alloc(&A.b.evb0, evb_bytes(A)));
+      if ((r = evb_copy(A, A.b.evb0, true))) return r;
+    }
+  }
+  CKA(A.b.alloc(&A.b.lr, sizeof(double)));
+  if (seg_k) {
     if (A.b.alloc(&A.b.stages, (size_t)seg_k * kord * bq) != cudaSuccess ||
         A.b.alloc(&A.b.traces, (size_t)seg_k * kord * bf) != cudaSuccess) {
       cudaGetLastError();
@@ -953,7 +1013,6 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
       A.b.traces = nullptr;
     }
   }
-  A.ckpt = snapshots > 0;
   const int nslots = seg_k ? nseg : snapshots;
   for (int s = 0; s < nslots; ++s) {
     double *p = nullptr, *pe = nullptr;
@@ -987,11 +1046,9 @@ extern "C" int dsem_adjoint(dsem_ctx *c, double dt, int nsteps, int window, int 
   }
   // ---- forward sweep
   std::vector<double> s_win;
-  const size_t npart = (size_t)c->ngrid * 5;
   if (window > 0) CKA(A.b.alloc(&A.b.eps_part, (size_t)window * npart * sizeof(double)));
   // the gradients saved by each window step's last stage, for the reverse
   // sweep's direct enstrophy term (else recomputed there)
-  const size_t nevb = (size_t)3 * c->nq;
   if (oop && !A.visc && window > 0 && !lean &&
       A.b.alloc(&A.b.evbw, (size_t)window * nevb * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();

@@ -104,7 +104,7 @@ struct dsem_ctx {
   bool keep_lob = false;  // the last stage of every step stores them (dsem_keep_lobatto)
   bool lob_valid = false; // QLB holds the arrays of the last stage run
   int adj_scheme = 0;     // dsem_adjoint with snapshots > 0: DSEM_ADJ_REVOLVE or DSEM_ADJ_SEGMENTS
-  cudaMemPool_t adj_pool = nullptr;  // dsem_adjoint's buffers (made by its first call)
+  cudaMemPool_t adj_pool = nullptr;  // dsem_adjoint's buffers when they are small
   cudaGraphExec_t gexec = nullptr;
   int graph_key = -1;
   long long graph_launches = 0;
