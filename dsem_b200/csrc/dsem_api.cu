@@ -1658,12 +1658,8 @@ int dsem_autotune(dsem_ctx *c, int reps, int *choice, double *ms) {
   CK(cudaEventCreate(&e1));
   for (auto &g : c->groups) {
     const int slot = g.G - 2;  // order p = G - 1 at index p - 1
-    int nv = 1;
-    CK(with_G(g.G, [&](auto gg) {
-      nv = Launch<decltype(gg)::value>::vol_variants();
-      return cudaSuccess;
-    }));
-    if (!g.diag || mode == VOL_EV || mode == VOL_EV_SAVE) nv = 1;  // shapes exist for the plain diagonal kernel
+    // shapes exist for the diagonal kernel without entropy viscosity
+    const int nv = g.diag && mode != VOL_EV && mode != VOL_EV_SAVE && vol_has_variants(g.G) ? VOL_VARIANTS : 1;
     const VolArgs a = vol_args(c, g);
     int best = 0;
     float tbest = 0.f;
@@ -1699,11 +1695,7 @@ int dsem_autotune(dsem_ctx *c, int reps, int *choice, double *ms) {
 
 int dsem_set_vol_variant(dsem_ctx *c, int p, int variant) {
   if (!c || p < 1 || p > DSEM_MAX_ORDER) return fail(c, DSEM_ERR_INVALID_ARG, "null context or order outside 1..8");
-  int nv = 1;
-  CK(with_G(p + 1, [&](auto gg) {
-    nv = Launch<decltype(gg)::value>::vol_variants();
-    return cudaSuccess;
-  }));
+  const int nv = vol_has_variants(p + 1) ? VOL_VARIANTS : 1;
   if (variant < 0 || variant >= nv) return fail(c, DSEM_ERR_INVALID_ARG, "no such launch shape for this order");
   c->vol_variant[p + 1] = variant;
   if (c->gexec) {

@@ -51,8 +51,8 @@ static cudaError_t vol_mma_one(const VolArgs &a, int nel, cudaStream_t s) {
 }
 
 // general metrics, p >= 3
-template <int G, bool MU, int SAVE, int V>
-static cudaError_t vol_gen_shape(const VolArgs &a, int nel, cudaStream_t s) {
+template <int G, bool MU, int SAVE, int V = MMA_GEN>
+static cudaError_t vol_gen_one(const VolArgs &a, int nel, cudaStream_t s) {
   using C = MmaCfg<G, V>;
   auto kern = k_vol_mma_gen<G, MU, SAVE, V>;
   static std::atomic<unsigned long long> attr{0};
@@ -62,67 +62,61 @@ static cudaError_t vol_gen_shape(const VolArgs &a, int nel, cudaStream_t s) {
   kern<<<nel, C::NT, C::SMEM, s>>>(a);
   return cudaGetLastError();
 }
-template <int G, bool MU, int SAVE> static cudaError_t vol_gen_one(const VolArgs &a, int nel, cudaStream_t s) {
-  if (G < 8 && nel <= 148 * MmaShape<G, MMA_GEN_WIDE>::MINB)  // (p >= 7: one element per SM anyway)
-    return vol_gen_shape<G, MU, SAVE, (G < 8 ? MMA_GEN_WIDE : MMA_GEN)>(a, nel, s);
-  return vol_gen_shape<G, MU, SAVE, MMA_GEN>(a, nel, s);
-}
 
-// launch shapes of k_vol_mma instantiated for this order (p = 4, 6, 8)
-template <int G> int Launch<G>::vol_variants() { return (G == 5 || G == 7 || G == 9) ? VOL_VARIANTS : 1; }
+// MU: with a viscosity model (entropy viscosity, Smagorinsky).  Entropy viscosity always saves the
+// temperature gradient too (SAVE = 2) and takes no explicit shape.
+template <int G, bool MU, int SAVE> static cudaError_t vol_mma_shape(const VolArgs &a, int nel, cudaStream_t s, int v) {
+  if constexpr (vol_has_variants(G) && SAVE != 2) {
+    switch (v) {
+      case 1: return vol_mma_one<G, MU, SAVE, 1>(a, nel, s);
+      case 2: return vol_mma_one<G, MU, SAVE, 2>(a, nel, s);
+      case 3: return vol_mma_one<G, MU, SAVE, 3>(a, nel, s);
+      case 4: return vol_mma_one<G, MU, SAVE, 4>(a, nel, s);
+    }
+  }
+  return v == MMA_WIDE ? vol_mma_one<G, MU, SAVE, MMA_WIDE>(a, nel, s) : vol_mma_one<G, MU, SAVE>(a, nel, s);
+}
+template <int G, bool MU, int SAVE> static cudaError_t vol_gen_shape(const VolArgs &a, int nel, cudaStream_t s, int v) {
+  if constexpr (G < 8)
+    if (v == MMA_GEN_WIDE) return vol_gen_one<G, MU, SAVE, MMA_GEN_WIDE>(a, nel, s);
+  return vol_gen_one<G, MU, SAVE>(a, nel, s);
+}
 
 template <int G>
 cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaStream_t s, int variant) {
-  if (diag) {
-    if constexpr (G >= 4) {
-      const bool ev = mode == VOL_EV || mode == VOL_EV_SAVE;
+  const bool ev = mode == VOL_EV || mode == VOL_EV_SAVE;
+  if constexpr (G >= 4) {
+    const int v = vol_shape(G, diag, nel, ev, a.nuhg != nullptr, variant);
+    if (diag) {
       VolArgs b = a;
       if (!ev) b.muhg = nullptr;
-      constexpr int W = MMA_WIDE;
-      const bool wide = nel <= 148 * MmaShape<G, W>::MINB, sv = mode == VOL_SAVE;
-      if (ev || a.nuhg) {  // with a viscosity model: the default shape
-        switch (mode) {
-          case VOL_SAVE: return wide ? vol_mma_one<G, true, 1, W>(b, nel, s) : vol_mma_one<G, true, 1>(b, nel, s);
-          case VOL_EV_SAVE: return wide ? vol_mma_one<G, true, 2, W>(b, nel, s) : vol_mma_one<G, true, 2>(b, nel, s);
-          default: return wide ? vol_mma_one<G, true, 0, W>(b, nel, s) : vol_mma_one<G, true, 0>(b, nel, s);
+      if (ev || a.nuhg) switch (mode) {
+          case VOL_SAVE: return vol_mma_shape<G, true, 1>(b, nel, s, v);
+          case VOL_EV_SAVE: return vol_mma_shape<G, true, 2>(b, nel, s, v);
+          default: return vol_mma_shape<G, true, 0>(b, nel, s, v);
         }
-      }
-      if constexpr (G == 5 || G == 7 || G == 9) {
-        switch (variant) {
-          case 1: return sv ? vol_mma_one<G, false, 1, 1>(b, nel, s) : vol_mma_one<G, false, 0, 1>(b, nel, s);
-          case 2: return sv ? vol_mma_one<G, false, 1, 2>(b, nel, s) : vol_mma_one<G, false, 0, 2>(b, nel, s);
-          case 3: return sv ? vol_mma_one<G, false, 1, 3>(b, nel, s) : vol_mma_one<G, false, 0, 3>(b, nel, s);
-          case 4: return sv ? vol_mma_one<G, false, 1, 4>(b, nel, s) : vol_mma_one<G, false, 0, 4>(b, nel, s);
-        }
-      }
-      if (wide) return sv ? vol_mma_one<G, false, 1, W>(b, nel, s) : vol_mma_one<G, false, 0, W>(b, nel, s);
-      if constexpr (G == 5)  // p = 4: between the two, four warps per element
-        if (nel <= 148 * MmaShape<G, 3>::MINB)
-          return sv ? vol_mma_one<G, false, 1, 3>(b, nel, s) : vol_mma_one<G, false, 0, 3>(b, nel, s);
-      return sv ? vol_mma_one<G, false, 1>(b, nel, s) : vol_mma_one<G, false, 0>(b, nel, s);
-    } else {
-      switch (mode) {
-        case VOL_SAVE: return vol_diag_one<G, false, 1>(a, nel, s);
-        case VOL_EV: return vol_diag_one<G, true, 0>(a, nel, s);
-        case VOL_EV_SAVE: return vol_diag_one<G, true, 2>(a, nel, s);
-        default: return vol_diag_one<G, false, 0>(a, nel, s);
-      }
+      return mode == VOL_SAVE ? vol_mma_shape<G, false, 1>(b, nel, s, v) : vol_mma_shape<G, false, 0>(b, nel, s, v);
     }
-  }
-  if constexpr (G >= VOL_GEN_GMIN) {
     switch (mode) {
-      case VOL_SAVE: return vol_gen_one<G, false, 1>(a, nel, s);
-      case VOL_EV: return vol_gen_one<G, true, 0>(a, nel, s);
-      case VOL_EV_SAVE: return vol_gen_one<G, true, 2>(a, nel, s);
-      default: return vol_gen_one<G, false, 0>(a, nel, s);
+      case VOL_SAVE: return vol_gen_shape<G, false, 1>(a, nel, s, v);
+      case VOL_EV: return vol_gen_shape<G, true, 0>(a, nel, s, v);
+      case VOL_EV_SAVE: return vol_gen_shape<G, true, 2>(a, nel, s, v);
+      default: return vol_gen_shape<G, false, 0>(a, nel, s, v);
+    }
+  } else if (diag) {
+    switch (mode) {
+      case VOL_SAVE: return vol_diag_one<G, false, 1>(a, nel, s);
+      case VOL_EV: return vol_diag_one<G, true, 0>(a, nel, s);
+      case VOL_EV_SAVE: return vol_diag_one<G, true, 2>(a, nel, s);
+      default: return vol_diag_one<G, false, 0>(a, nel, s);
     }
   } else {
-  switch (mode) {
-    case VOL_SAVE: return vol_one<G, false, 1>(a, nel, s);
-    case VOL_EV: return vol_one<G, true, 0>(a, nel, s);
-    case VOL_EV_SAVE: return vol_one<G, true, 2>(a, nel, s);
-    default: return vol_one<G, false, 0>(a, nel, s);
-  }
+    switch (mode) {
+      case VOL_SAVE: return vol_one<G, false, 1>(a, nel, s);
+      case VOL_EV: return vol_one<G, true, 0>(a, nel, s);
+      case VOL_EV_SAVE: return vol_one<G, true, 2>(a, nel, s);
+      default: return vol_one<G, false, 0>(a, nel, s);
+    }
   }
 }
 

@@ -5,6 +5,8 @@
 
 #include <atomic>
 
+#include "dsem_shapes.h"
+
 namespace dsem {
 
 struct Phys;
@@ -36,17 +38,10 @@ cudaError_t set_smem_once(K kern, size_t smem, std::atomic<unsigned long long> &
 
 // volume kernel variants: metric layout x entropy viscosity x saved gradients
 enum VolMode { VOL_PLAIN = 0, VOL_SAVE = 1, VOL_EV = 2, VOL_EV_SAVE = 3 };
-// launch shapes of the diagonal volume kernel the autotuner chooses from
-constexpr int VOL_VARIANTS = 5;
-
-// smallest G = p + 1 whose elements with full metrics run k_vol_mma_gen
-constexpr int VOL_GEN_GMIN = 4;
-
 template <int G> struct Launch {
   static cudaError_t set_ops(const double *host_ops, int n);  // copies the operator table to constant memory
   // (with a.JQ null: only the kernel's attributes are set, for the shape of nel elements)
   static cudaError_t vol(const VolArgs &a, int nel, bool diag, int mode, cudaStream_t s, int variant = 0);
-  static int vol_variants();                // launch shapes available for this order (1 or VOL_VARIANTS)
   static cudaError_t update(const UpdArgs &a, int nel, cudaStream_t s);
   static cudaError_t trace(const TraceArgs &a, int nel, cudaStream_t s);
   // Lobatto arrays of the stage kept in a.QLB; gradients rebuilt from them into a.EVB

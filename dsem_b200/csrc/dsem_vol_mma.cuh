@@ -33,6 +33,7 @@
 // 20^3: 1.286 -> 0.492; p = 6, 24^3: 1.088 -> 0.745; p = 5, 24^3: 0.568 -> 0.526;
 // p = 4, 32^3: 0.716 -> 0.640; p = 3, 32^3: 0.371 -> 0.299.
 #pragma once
+#include "dsem_shapes.h"
 #include "dsem_stage.cuh"
 
 namespace dsem {
@@ -54,35 +55,6 @@ __host__ __device__ constexpr int mma_plane(int G) {
   return s;
 }
 
-// Launch shapes: warps per element (NW) and the elements an SM must hold at once
-// (MINB, which sets the register budget).  Variant 0 is the default; dsem_autotune times
-// 1..4 against it for p = 4, 6, 8.  Shared memory allows 2 elements per SM at p >= 7, 4 at
-// p = 6, 6 at p = 5 and 10 at p = 4.  Measured, ms of variants 0..4 (22^3 of p = 8, 24^3 of
-// p = 6, 32^3 of p = 4): 1.127 1.156 1.180 1.233 1.307; 0.745 0.762 0.946 0.739 0.854;
-// 0.640 0.708 0.644 0.700 0.671.  Every shape evaluates each value with the same chain.
-// MMA_GEN, MMA_GEN_WIDE: k_vol_mma_gen's shapes (20 shared fields).
-// MMA_WIDE: the shape of variant 0 for launches of at most 148 * MINB elements, which do
-// not fill the GPU: more warps work on one element, and its latency is the launch's.
-// Measured against variant 1's or 0's shape, us: 4^3 elements of p = 8 23.8 (8 warps: 27),
-// p = 6 15.6 (3 warps: 24.7), p = 4 10.4 (2 warps: 16.5); p = 4 at 512 elements, which
-// variant 3 still holds at once, 16.5 with it (2 warps: 19.6).
-constexpr int MMA_WIDE = 5, MMA_GEN = 6, MMA_GEN_WIDE = 7;
-template <int G, int V> struct MmaShape {
-  static constexpr bool W = V == MMA_WIDE, GEN = V == MMA_GEN, GW = V == MMA_GEN_WIDE;
-  static constexpr int NW = GEN ? (G >= 8 ? 12 : (G == 7 ? 4 : 2))
-                          : GW ? (G >= 7 ? 12 : (G == 6 ? 8 : 4))
-                          : G >= 8 ? (W ? 16 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 7 : (V == 3 ? 5 : 4)))))
-                          : G >= 6 ? (W ? (G == 7 ? 12 : 8) : (V == 0 ? 4 : (V == 1 ? 3 : (V == 2 ? 2 : (V == 3 ? 5 : 6)))))
-                          : G == 5 ? (W ? 8 : (V <= 2 ? 2 : (V == 3 ? 4 : 3)))
-                                   : (W ? 4 : 2);
-  static constexpr int MINB = GEN ? (G >= 8 ? 1 : (G == 7 ? 3 : (G == 6 ? 6 : 8)))
-                            : GW ? (G >= 7 ? 1 : (G == 6 ? 1 : 3))
-                            : G >= 8 ? (W ? 1 : 2)
-                            : G >= 6 ? (W ? (G == 7 ? 1 : 2) : (V == 3 ? 3 : (V == 4 ? 2 : 4)))
-                            : G == 5 ? (W ? 2 : (V == 0 ? 8 : (V == 1 ? 6 : (V == 2 ? 10 : (V == 3 ? 4 : 5)))))
-                                     : (W ? 4 : 8);
-};
-
 template <int G, int V> struct MmaCfg {
   static constexpr int L = G + 1, G2 = G * G, NG = G * G * G, NL = L * G * G;
   static constexpr int PS = mma_plane(G), FS = G * PS;  // padded plane and field strides
@@ -93,8 +65,8 @@ template <int G, int V> struct MmaCfg {
   static constexpr int KS = KR == 3 ? 0 : KR;           // k on scalar FMAs
   static constexpr int NTILE = (G2 + 7) / 8;            // tiles of 8 lines per direction
   static constexpr int NLW = (G2 + 31) / 32;            // warps of one line per lane
-  static constexpr int NW = MmaShape<G, V>::NW, NT = 32 * NW;
-  static constexpr int MINB = MmaShape<G, V>::MINB;
+  static constexpr int NW = mma_warps(G, V), NT = 32 * NW;
+  static constexpr int MINB = mma_minb(G, V);
   // shared fields: state 5, gradients of fields 0..3 12, energy gradient 2 buffers (general metrics: 5, 15)
   static constexpr int NF = V == MMA_GEN || V == MMA_GEN_WIDE ? 20 : 19;
   static constexpr size_t SMEM = sizeof(double) * (size_t)(NF * FS) + 16;

@@ -179,8 +179,10 @@ int dsem_load_state(dsem_ctx *ctx, const void *buf, long long nbytes);
  * element order of the context, times the launch shapes of the volume kernel
  * (threads per element, elements held per SM) on the context's own elements
  * and current state, `reps` launches each, and keeps the fastest for the
- * following steps.  Shapes exist for p = 4, 6 and 8 (other orders have one);
- * all give identical results.  choice[p-1] receives the chosen shape of order p
+ * following steps.  Shapes exist for p = 4, 6 and 8 on axis-aligned elements,
+ * without a model and with Smagorinsky's (other orders, full metrics and
+ * entropy viscosity have one, whatever variant is set); all give identical
+ * results.  choice[p-1] receives the chosen shape of order p
  * and ms[(p-1)*DSEM_VOL_VARIANTS + v] the mean time of shape v (-1: not timed);
  * either may be NULL.  Call it after dsem_upload_q.  dsem_set_vol_variant
  * sets a shape by hand. */

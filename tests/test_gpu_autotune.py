@@ -88,3 +88,26 @@ def test_shape_arguments_are_checked():
         s.set_vol_variant(4, 5)
     s.set_vol_variant(4, 4)  # an order the context does not use: accepted, unused
     s.close()
+
+
+@pytest.mark.parametrize("p", [4, 6, 8])
+def test_every_launch_shape_with_the_smagorinsky_model(p):
+    """The shapes serve runs with the Smagorinsky model too, and the tuner times all of them."""
+    from dsem_b200.solver import Solver
+    box = mesh.Box(3, 2, 2, p)
+    q = mesh.random_isotropic(box, seed=p, k0=2.0, mach_t=0.3)
+    dt = 0.3 * mesh.dtcalc(box, q)
+    ref = None
+    for v in range(5):
+        s = Solver(box.desc(), re=900.0)
+        s.set_les(0.1, 1e3)
+        s.upload(q)
+        s.set_vol_variant(p, v)
+        s.diag(dt, first=True)  # the steps save their gradients
+        s.step(dt, 2)
+        out = (s.download(), s.rhs())
+        ref = ref or out
+        assert all(np.array_equal(a, b) for a, b in zip(out, ref)), v
+        choice, ms = s.autotune(reps=2)
+        assert 0 <= choice[p] < 5 and np.all(ms[p - 1] > 0)
+        s.close()
