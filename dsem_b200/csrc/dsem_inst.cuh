@@ -64,7 +64,7 @@ static cudaError_t vol_gen_one(const VolArgs &a, int nel, cudaStream_t s) {
 }
 
 // MU: with a viscosity model (entropy viscosity, Smagorinsky).  Entropy viscosity always saves the
-// temperature gradient too (SAVE = 2) and takes no explicit shape.
+// temperature gradient too (SAVE = 2) and takes no explicit shape, but the default rule's shape 3 at p = 4.
 template <int G, bool MU, int SAVE> static cudaError_t vol_mma_shape(const VolArgs &a, int nel, cudaStream_t s, int v) {
   if constexpr (vol_has_variants(G) && SAVE != 2) {
     switch (v) {
@@ -74,6 +74,8 @@ template <int G, bool MU, int SAVE> static cudaError_t vol_mma_shape(const VolAr
       case 4: return vol_mma_one<G, MU, SAVE, 4>(a, nel, s);
     }
   }
+  if constexpr (G == 5 && SAVE == 2)
+    if (v == 3) return vol_mma_one<G, MU, SAVE, 3>(a, nel, s);
   return v == MMA_WIDE ? vol_mma_one<G, MU, SAVE, MMA_WIDE>(a, nel, s) : vol_mma_one<G, MU, SAVE>(a, nel, s);
 }
 template <int G, bool MU, int SAVE> static cudaError_t vol_gen_shape(const VolArgs &a, int nel, cudaStream_t s, int v) {
@@ -86,7 +88,7 @@ template <int G>
 cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaStream_t s, int variant) {
   const bool ev = mode == VOL_EV || mode == VOL_EV_SAVE;
   if constexpr (G >= 4) {
-    const int v = vol_shape(G, diag, nel, ev, a.nuhg != nullptr, variant);
+    const int v = vol_shape(G, diag, nel, ev, variant);
     if (diag) {
       VolArgs b = a;
       if (!ev) b.muhg = nullptr;

@@ -19,7 +19,8 @@ constexpr int VOL_VARIANTS = 5;
 // fill the GPU: more warps work on one element, and its latency is the launch's.  Measured against
 // variant 1's or 0's shape, us: 4^3 elements of p = 8 23.8 (8 warps: 27), p = 6 15.6 (3 warps:
 // 24.7), p = 4 10.4 (2 warps: 16.5); p = 4 at 512 elements, which shape 3 still holds at
-// once, 16.5 with it (2 warps: 19.6).
+// once, 16.5 with it (2 warps: 19.6); a step of 343 elements with a viscosity model 121.2 us
+// against 147.9 (Smagorinsky), 125.2 against 153.8 (entropy viscosity).
 // MMA_GEN, MMA_GEN_WIDE: k_vol_mma_gen (20 shared fields), the latter for the same reason.
 constexpr int MMA_WIDE = 5, MMA_GEN = 6, MMA_GEN_WIDE = 7;
 constexpr int mma_warps(int G, int V) {
@@ -46,13 +47,13 @@ constexpr bool vol_has_variants(int G) { return G == 5 || G == 7 || G == 9; }
 // kernels with a thread per point (k_vol_diag, k_vol): p = 1, 2, whose lines are too few for the
 // 8-line tiles.  ev: entropy viscosity (its launches have the default shapes only).
 constexpr int VOL_POINT = -1;
-constexpr int vol_shape(int G, bool diag, int nel, bool ev, bool les, int variant) {
+constexpr int vol_shape(int G, bool diag, int nel, bool ev, int variant) {
   if (G < 4) return VOL_POINT;
   if (!diag)  // (p >= 7: one element per SM in either shape)
     return G < 8 && nel <= SM_COUNT * mma_minb(G, MMA_GEN_WIDE) ? MMA_GEN_WIDE : MMA_GEN;
   if (variant > 0 && variant < VOL_VARIANTS && vol_has_variants(G) && !ev) return variant;
   if (nel <= SM_COUNT * mma_minb(G, MMA_WIDE)) return MMA_WIDE;
-  if (G == 5 && !ev && !les && nel <= SM_COUNT * mma_minb(G, 3)) return 3;  // p = 4: between the two, four warps
+  if (G == 5 && nel <= SM_COUNT * mma_minb(G, 3)) return 3;  // p = 4: between the two, four warps
   return 0;
 }
 

@@ -11,14 +11,14 @@ WIDE, GEN, GEN_WIDE, POINT = 5, 6, 7, -1
 
 @pytest.fixture(scope="module")
 def shape(tmp_path_factory):
-    """shape([(G, diag, nel, ev, les, variant), ...]) -> the shapes."""
+    """shape([(G, diag, nel, ev, variant), ...]) -> the shapes."""
     if not shutil.which("g++"):
         pytest.skip("no host C++ compiler")
     d = tmp_path_factory.mktemp("shapes")
     src, exe = d / "shapes.cpp", d / "shapes"
-    src.write_text('#include <cstdio>\n#include "dsem_shapes.h"\nint main() {\n  int g, d, n, e, l, v;\n'
-                   '  while (std::scanf("%d%d%d%d%d%d", &g, &d, &n, &e, &l, &v) == 6)\n'
-                   '    std::printf("%d\\n", dsem::vol_shape(g, d != 0, n, e != 0, l != 0, v));\n}\n')
+    src.write_text('#include <cstdio>\n#include "dsem_shapes.h"\nint main() {\n  int g, d, n, e, v;\n'
+                   '  while (std::scanf("%d%d%d%d%d", &g, &d, &n, &e, &v) == 5)\n'
+                   '    std::printf("%d\\n", dsem::vol_shape(g, d != 0, n, e != 0, v));\n}\n')
     r = subprocess.run(["g++", "-std=c++17", "-Wall", "-Wextra", "-Werror", "-I", CSRC, str(src), "-o", str(exe)],
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
@@ -37,10 +37,16 @@ def test_explicit_shapes(shape, p):
     G = p + 1
     for nel in (1, 200, 5000):
         for v in range(1, 5):
-            for les in (0, 1):
-                plain, default = shape([(G, 1, nel, 0, les, v), (G, 1, nel, 0, les, 0)])
-                assert plain == (v if p in (4, 6, 8) else default)
-                ev, evd = shape([(G, 1, nel, 1, les, v), (G, 1, nel, 1, les, 0)])
-                assert ev == evd
-            gen, gend = shape([(G, 0, nel, 0, 0, v), (G, 0, nel, 0, 0, 0)])
+            plain, default = shape([(G, 1, nel, 0, v), (G, 1, nel, 0, 0)])
+            assert plain == (v if p in (4, 6, 8) else default)
+            ev, evd = shape([(G, 1, nel, 1, v), (G, 1, nel, 1, 0)])
+            assert ev == evd
+            gen, gend = shape([(G, 0, nel, 0, v), (G, 0, nel, 0, 0)])
             assert gen == gend
+
+
+@pytest.mark.parametrize("ev", [0, 1])
+def test_default_shape_at_p4(shape, ev):
+    """p = 4, with a model as without: wide up to 2 elements per SM, four warps up to 4, two above."""
+    rows = [(5, 1, n, ev, 0) for n in (1, 296, 297, 592, 593)]
+    assert shape(rows) == [WIDE, WIDE, 3, 3, 0]
