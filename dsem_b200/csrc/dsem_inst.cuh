@@ -13,7 +13,7 @@ template <int G> cudaError_t Launch<G>::set_ops(const double *h, int n) {
   return cudaMemcpyToSymbol(c_ops, h, sizeof(double) * OPS_TOTAL);
 }
 
-// general metrics, p = 1, 2
+// general metrics, p = 1, 2, and small launches at p = 4, 5
 template <int G, bool EV, int SAVE> static cudaError_t vol_one(const VolArgs &a, int nel, cudaStream_t s) {
   using C = VolCfg<G, EV>;
   auto kern = k_vol<G, EV, SAVE>;
@@ -99,6 +99,13 @@ cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaS
         }
       return mode == VOL_SAVE ? vol_mma_shape<G, false, 1>(b, nel, s, v) : vol_mma_shape<G, false, 0>(b, nel, s, v);
     }
+    if constexpr (vol_point_max(G) > 0)
+      if (v == VOL_POINT) switch (mode) {
+          case VOL_SAVE: return vol_one<G, false, 1>(a, nel, s);
+          case VOL_EV: return vol_one<G, true, 0>(a, nel, s);
+          case VOL_EV_SAVE: return vol_one<G, true, 2>(a, nel, s);
+          default: return vol_one<G, false, 0>(a, nel, s);
+        }
     switch (mode) {
       case VOL_SAVE: return vol_gen_shape<G, false, 1>(a, nel, s, v);
       case VOL_EV: return vol_gen_shape<G, true, 0>(a, nel, s, v);

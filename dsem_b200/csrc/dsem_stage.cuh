@@ -820,7 +820,8 @@ struct VolArgs {
 };
 
 // k_vol: full metrics (rotated, skewed or curved elements) at p = 1, 2, whose lines are too
-// few for the tiles of k_vol_mma_gen.
+// few for the tiles of k_vol_mma_gen, and at p = 4, 5 for launches that leave an SM one element
+// (vol_point_max).
 template <int G, bool EV> struct VolCfg {
   static constexpr int L = G + 1, NG = G * G * G;
   static constexpr int NCH = 15;              // gradient fields interpolated to each grid

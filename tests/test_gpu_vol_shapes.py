@@ -33,3 +33,11 @@ def _check(oracle_mod, box, model):
 @pytest.mark.parametrize("model", ["none", "ev", "les", "ev+les"])
 def test_p4_between_two_and_four_elements_per_sm(oracle_mod, model):
     _check(oracle_mod, mesh.Box(10, 6, 5, 4), model)  # 300 elements
+
+
+@pytest.mark.parametrize("model", ["none", "ev"])
+@pytest.mark.parametrize("p,n", [(4, (7, 7, 3)), (4, (6, 5, 5)), (4, (8, 8, 7)), (5, (7, 6, 7)), (5, (10, 6, 5)),
+                                 (5, (8, 8, 7))])
+def test_full_metrics_at_p4_and_p5(oracle_mod, p, n, model):
+    """Each side of the limits at 148 (p = 4), 296 (p = 5) and 444 elements."""
+    _check(oracle_mod, mesh.Box(*n, p, warp=0.02), model)

@@ -50,3 +50,11 @@ def test_default_shape_at_p4(shape, ev):
     """p = 4, with a model as without: wide up to 2 elements per SM, four warps up to 4, two above."""
     rows = [(5, 1, n, ev, 0) for n in (1, 296, 297, 592, 593)]
     assert shape(rows) == [WIDE, WIDE, 3, 3, 0]
+
+
+@pytest.mark.parametrize("p,limits", [(3, (0, 444)), (4, (148, 444)), (5, (296, 444)), (6, (0, 148))])
+def test_shapes_of_full_metrics(shape, p, limits):
+    """Small launches at p = 4, 5 run the kernel with a thread per point, then the wide shape."""
+    point, wide = limits
+    rows = [(p + 1, 0, n, ev, 0) for ev in (0, 1) for n in (max(point, 1), point + 1, wide, wide + 1)]
+    assert shape(rows) == 2 * [POINT if point else GEN_WIDE, GEN_WIDE, GEN_WIDE, GEN]
