@@ -950,9 +950,9 @@ __device__ __forceinline__ void vol_dir(const VolArgs &A, const double *JQ, cons
       Qz[v] = CH[(v * 3 + 2) * NLS + p];
     }
     double f[NV], g[NV], h[NV];
-    vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, f);
-    vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, g);
-    vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, h);
+    vis_flux_x<EV>(Q, rr, Qx, Qy, Qz, amu, P, f);
+    vis_flux_y<EV>(Q, rr, Qx, Qy, Qz, amu, P, g);
+    vis_flux_z<EV>(Q, rr, Qx, Qy, Qz, amu, P, h);
     const double *g3 = gm + ((long long)D * NL + qi) * 3;
     const double m0 = g3[0], m1 = g3[1], m2 = g3[2];
 #pragma unroll

@@ -144,17 +144,17 @@ __device__ __forceinline__ void vol_diag_point(int qi, int s, int a, int b, cons
     Qx[0] = c[0]; Qx[1] = c[1]; Qx[2] = c[2]; Qx[3] = c[3]; Qx[4] = c[4];
     Qy[0] = c[5]; Qy[1] = c[6]; Qy[2] = c[7]; Qy[3] = 0.0; Qy[4] = 0.0;
     Qz[0] = c[8]; Qz[1] = c[9]; Qz[3] = c[10]; Qz[2] = 0.0; Qz[4] = 0.0;
-    vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_x<true>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   } else if (D == 1) {
     Qy[0] = c[0]; Qy[1] = c[1]; Qy[2] = c[2]; Qy[3] = c[3]; Qy[4] = c[4];
     Qx[0] = c[5]; Qx[1] = c[6]; Qx[2] = c[7]; Qx[3] = 0.0; Qx[4] = 0.0;
     Qz[0] = c[8]; Qz[2] = c[9]; Qz[3] = c[10]; Qz[1] = 0.0; Qz[4] = 0.0;
-    vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_y<true>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   } else {
     Qz[0] = c[0]; Qz[1] = c[1]; Qz[2] = c[2]; Qz[3] = c[3]; Qz[4] = c[4];
     Qx[0] = c[5]; Qx[1] = c[6]; Qx[3] = c[7]; Qx[2] = 0.0; Qx[4] = 0.0;
     Qy[0] = c[8]; Qy[2] = c[9]; Qy[3] = c[10]; Qy[1] = 0.0; Qy[4] = 0.0;
-    vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_z<true>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) r[v] = gdiag * fl[v];

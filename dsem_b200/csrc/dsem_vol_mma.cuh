@@ -123,7 +123,7 @@ template <int G, int D> __device__ __forceinline__ constexpr int mma_stride() {
 
 // Viscous flux of direction D times gdiag into r from the point's state and its
 // 11 interpolated gradient fields (diag_field order).
-template <int D>
+template <int D, bool MU>
 __device__ __forceinline__ void mma_vis(const double *Q, double rr, const double *c, double amu, double gdiag,
                                         const Phys &P, double *r) {
   double Qx[NV], Qy[NV], Qz[NV], fl[NV];
@@ -131,17 +131,17 @@ __device__ __forceinline__ void mma_vis(const double *Q, double rr, const double
     Qx[0] = c[0]; Qx[1] = c[1]; Qx[2] = c[2]; Qx[3] = c[3]; Qx[4] = c[4];
     Qy[0] = c[5]; Qy[1] = c[6]; Qy[2] = c[7]; Qy[3] = 0.0; Qy[4] = 0.0;
     Qz[0] = c[8]; Qz[1] = c[9]; Qz[3] = c[10]; Qz[2] = 0.0; Qz[4] = 0.0;
-    vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_x<MU>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   } else if (D == 1) {
     Qy[0] = c[0]; Qy[1] = c[1]; Qy[2] = c[2]; Qy[3] = c[3]; Qy[4] = c[4];
     Qx[0] = c[5]; Qx[1] = c[6]; Qx[2] = c[7]; Qx[3] = 0.0; Qx[4] = 0.0;
     Qz[0] = c[8]; Qz[2] = c[9]; Qz[3] = c[10]; Qz[1] = 0.0; Qz[4] = 0.0;
-    vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_y<MU>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   } else {
     Qz[0] = c[0]; Qz[1] = c[1]; Qz[2] = c[2]; Qz[3] = c[3]; Qz[4] = c[4];
     Qx[0] = c[5]; Qx[1] = c[6]; Qx[3] = c[7]; Qx[2] = 0.0; Qx[4] = 0.0;
     Qy[0] = c[8]; Qy[2] = c[9]; Qy[3] = c[10]; Qy[1] = 0.0; Qy[4] = 0.0;
-    vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_z<MU>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) r[v] = gdiag * fl[v];
@@ -295,7 +295,7 @@ __device__ __forceinline__ void mma_tile(int t, const MmaOps<G, V> &O, const Phy
     if (ev) amu = amu + mu[i];
     const double rr = 1.0 / Q[i][0];
     double r[NV], fi[NV];
-    mma_vis<D>(Q[i], rr, c[i], amu, gd[i], P, r);
+    mma_vis<D, MU>(Q[i], rr, c[i], amu, gd[i], P, r);
     euler_flux(D, Q[i], rr, P.gm1, fi);
     const bool in = (i == 0 ? 1 : 5) + q <= C::NS;  // padded points contribute exact zeros
 #pragma unroll
@@ -349,7 +349,7 @@ __device__ __forceinline__ void mma_faces(int ln, const Phys &P, const double *Q
     double amu = 1.0;
     if (les) amu = amu + nu[i] * Q[i][0];
     if (ev) amu = amu + mu[i];
-    mma_vis<D>(Q[i], 1.0 / Q[i][0], c[i], amu, gd[i], P, r);
+    mma_vis<D, MU>(Q[i], 1.0 / Q[i][0], c[i], amu, gd[i], P, r);
     double *o = VF + ((i ? face_hi(D) : face_lo(D)) - 1) * 5 * G2 + ln;
 #pragma unroll
     for (int v = 0; v < NV; ++v) o[v * G2] = r[v];
@@ -600,7 +600,7 @@ __device__ __forceinline__ void mma_gen_grad(int t, const MmaOps<G, V> &O, const
 }
 
 // r = m . (viscous fluxes), and with INV also e = m . (Euler fluxes) at one point.
-template <bool INV>
+template <bool INV, bool MU>
 __device__ __forceinline__ void mma_gen_flux(const double *Q, const double *c, const double *m, double amu,
                                              const Phys &P, double *r, double *e) {
   double Qx[NV], Qy[NV], Qz[NV], f[NV], g[NV], h[NV];
@@ -611,9 +611,9 @@ __device__ __forceinline__ void mma_gen_flux(const double *Q, const double *c, c
     Qz[v] = c[v * 3 + 2];
   }
   const double rr = 1.0 / Q[0];
-  vis_flux_x(Q, rr, Qx, Qy, Qz, amu, P, f);
-  vis_flux_y(Q, rr, Qx, Qy, Qz, amu, P, g);
-  vis_flux_z(Q, rr, Qx, Qy, Qz, amu, P, h);
+  vis_flux_x<MU>(Q, rr, Qx, Qy, Qz, amu, P, f);
+  vis_flux_y<MU>(Q, rr, Qx, Qy, Qz, amu, P, g);
+  vis_flux_z<MU>(Q, rr, Qx, Qy, Qz, amu, P, h);
 #pragma unroll
   for (int v = 0; v < NV; ++v) r[v] = m[0] * f[v] + m[1] * g[v] + m[2] * h[v];
   if (INV) {
@@ -655,7 +655,7 @@ __device__ __forceinline__ void mma_gen_tile(int t, const MmaOps<G, V> &O, const
   for (int i = 0; i < C::NI; ++i) {
     double amu = 1.0, r[NV], e[NV];
     if (MU) amu = amu + mu[i];
-    mma_gen_flux<true>(Q[i], c[i], m[i], amu, P, r, e);
+    mma_gen_flux<true, MU>(Q[i], c[i], m[i], amu, P, r, e);
     const bool in = (i == 0 ? 1 : 5) + q <= C::NS;
 #pragma unroll
     for (int v = 0; v < NV; ++v) f[i][v] = in ? e[v] - ddiv(r[v], P.re, P.r_re) : 0.0;
@@ -688,7 +688,7 @@ __device__ __forceinline__ void mma_gen_face(int ln, const Phys &P, const double
   for (int j = 0; j < 15; ++j) c[j] = end(GR + j * FS + pl, S);
   double amu = 1.0;
   if (MU) amu = amu + end(muhg + gbase<G>(D, a, b), xs);
-  mma_gen_flux<false>(Q, c, m, amu, P, r, nullptr);
+  mma_gen_flux<false, MU>(Q, c, m, amu, P, r, nullptr);
 #pragma unroll
   for (int v = 0; v < NV; ++v) VF[o + v * G2] = r[v];
 }
