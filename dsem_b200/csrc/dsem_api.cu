@@ -131,6 +131,23 @@ int cuda_fail(dsem_ctx *c, cudaError_t e, const char *where) {
     if (e_ != cudaSuccess) return cuda_fail(c, e_, #call); \
   } while (0)
 
+// Sets the shared-memory attributes of the volume kernels that group g's launches take in its
+// present shape, in every mode and with the Smagorinsky model, so that none is set inside a
+// capture.
+cudaError_t prepare_vol(const dsem_ctx *c, const Group &g) {
+  const double model = 0.0;  // stands for a viscosity array: nothing is launched
+  for (int mode = 0; mode < 4; ++mode)
+    for (int les = 0; les < (g.diag ? 2 : 1); ++les) {
+      VolArgs a{};
+      if (les) a.nuhg = &model;
+      const cudaError_t e = with_G(g.G, [&](auto gg) {
+        return Launch<decltype(gg)::value>::vol(a, g.nel, g.diag, mode, c->st, c->vol_variant[g.G]);
+      });
+      if (e != cudaSuccess) return e;
+    }
+  return cudaSuccess;
+}
+
 // diagnostic sums of group g's elements from state jq and gradients evb into part
 cudaError_t launch_diag(const dsem_ctx *c, const Group &g, const double *jq, const double *evb, bool have,
                         double *part) {
@@ -1141,12 +1158,7 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
       }
     }
   }
-  // set the shared-memory attribute of every volume variant outside any capture
-  for (auto &g : c->groups)
-    for (int mode = 0; mode < 4; ++mode) {
-      VolArgs a{};  // no state: nothing is launched
-      CK(with_G(g.G, [&](auto gg) { return Launch<decltype(gg)::value>::vol(a, g.nel, g.diag, mode, c->st); }));
-    }
+  for (auto &g : c->groups) CK(prepare_vol(c, g));
   return DSEM_OK;
 }
 
@@ -1683,6 +1695,7 @@ int dsem_autotune(dsem_ctx *c, int reps, int *choice, double *ms) {
     }
     c->vol_variant[g.G] = best;
     if (choice) choice[slot] = best;
+    CK(prepare_vol(c, g));
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1698,6 +1711,8 @@ int dsem_set_vol_variant(dsem_ctx *c, int p, int variant) {
   const int nv = vol_has_variants(p + 1) ? VOL_VARIANTS : 1;
   if (variant < 0 || variant >= nv) return fail(c, DSEM_ERR_INVALID_ARG, "no such launch shape for this order");
   c->vol_variant[p + 1] = variant;
+  for (auto &g : c->groups)
+    if (g.G == p + 1) CK(prepare_vol(c, g));
   if (c->gexec) {
     cudaGraphExecDestroy(c->gexec);
     c->gexec = nullptr;

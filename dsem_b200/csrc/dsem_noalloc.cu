@@ -25,6 +25,7 @@
 //    returning.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -64,6 +65,9 @@ template <class F> cudaError_t with_G(int G, F &&f) {
   }
 }
 
+// doubles of the scratch array that nel elements of G = p + 1 need
+long long scratch_doubles(int G, long long nel) { return nel * (90LL * G * G + 5LL * G * G * G) + 1; }
+
 // Per-device set-up, once, with the device current.  Returns the device
 // address of the scratch array (the host-side name g_noalloc_scratch is only a
 // stand-in and must never be passed to a kernel).
@@ -86,9 +90,16 @@ int setup_device(int dev, double **out) {
   for (int G = GMIN; G <= GMAX; ++G) {
     e = with_G(G, [&](auto g) { return Launch<decltype(g)::value>::set_ops(table.data(), OPS_TOTAL); });
     if (e != cudaSuccess) return nfail(DSEM_ERR_CUDA, std::string("operator tables: ") + cudaGetErrorString(e));
-    VolArgs a{};
-    e = with_G(G, [&](auto g) { return Launch<decltype(g)::value>::vol(a, 0, true, VOL_PLAIN, nullptr); });
-    if (e != cudaSuccess) return nfail(DSEM_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
+    // the volume kernel in every shape that a mesh within the scratch array can take
+    int last = INT_MAX;
+    for (int nel = 1; scratch_doubles(G, nel) <= DSEM_NOALLOC_SCRATCH_DOUBLES; ++nel) {
+      const int shape = vol_shape(G, true, nel, false, 0);
+      if (shape == last) continue;
+      last = shape;
+      VolArgs a{};
+      e = with_G(G, [&](auto g) { return Launch<decltype(g)::value>::vol(a, nel, true, VOL_PLAIN, nullptr); });
+      if (e != cudaSuccess) return nfail(DSEM_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
+    }
   }
   g_scratch_ptr[dev] = ptr;
   *out = ptr;
@@ -259,7 +270,7 @@ int dsem_rhs_noalloc(int nel, int p, int nmort, const int *mortar, const double 
   if (nel <= 0 || nmort < 0) return nfail(DSEM_ERR_INVALID_ARG, "dsem_rhs_noalloc: bad element or mortar count");
   if (!JQ || !jac || !gmetg_diag || !gmet_diag || !Qt || (nmort > 0 && (!mortar || !n_hat || !norm)))
     return nfail(DSEM_ERR_INVALID_ARG, "dsem_rhs_noalloc: null device pointer");
-  const long long need = (long long)nel * (90LL * G * G + 5LL * G * G * G) + 1;
+  const long long need = scratch_doubles(G, nel);
   if (need > (long long)DSEM_NOALLOC_SCRATCH_DOUBLES)
     return nfail(DSEM_ERR_INVALID_ARG,
                  "dsem_rhs_noalloc: mesh too large for the static scratch (" + std::to_string(need) +

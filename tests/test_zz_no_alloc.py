@@ -126,3 +126,20 @@ def test_noalloc_rejects_nonconforming_rows(lib, field, value):
     assert b"conforming" in lib.dsem_last_error(None)
     rc, _ = call_noalloc(lib, box, internal_arrays(box, mesh.taylor_green(box)), torch, 3)
     assert rc == 0
+
+
+@pytest.mark.parametrize("n,p", [((11, 9, 6), 3), ((7, 7, 7), 4), ((6, 5, 5), 6)])
+def test_noalloc_takes_every_launch_shape(lib, n, p):
+    """Meshes near the scratch array's limit, whose volume launches take other shapes than small ones."""
+    import torch
+    from dsem_b200.solver import Solver
+    box = mesh.Box(*n, p)
+    q = mesh.perturbed_taylor_green(box, seed=p, amp=0.2)
+    s = Solver(box.desc(), re=1600.0)
+    s.upload(q)
+    G = p + 1
+    ref = s.rhs()[:, :, :G, :G, :G]
+    s.close()
+    rc, got = call_noalloc(lib, box, internal_arrays(box, q), torch, p)
+    assert rc == 0, lib.dsem_last_error(None)
+    assert float(np.abs(got - ref).max() / np.abs(ref).max()) <= RHS_TOL
