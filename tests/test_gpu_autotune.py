@@ -111,3 +111,15 @@ def test_every_launch_shape_with_the_smagorinsky_model(p):
         choice, ms = s.autotune(reps=2)
         assert 0 <= choice[p] < 5 and np.all(ms[p - 1] > 0)
         s.close()
+
+
+@pytest.mark.parametrize("p,n", [(4, (10, 10, 6)), (6, (6, 5, 5)), (8, (6, 5, 5))])
+def test_every_launch_shape_on_full_launches(p, n):
+    """The same where variant 0 is shape 0 (above 592, 148 and 148 elements; a smaller launch's
+    variant 0 is the wide shape)."""
+    box = mesh.Box(*n, p)
+    q = mesh.random_isotropic(box, seed=p, k0=2.0, mach_t=0.3)
+    dt = 0.3 * mesh.dtcalc(box, q)
+    ref = _run(box, q, dt, variant=0)
+    for v in (1, 2, 3, 4):
+        assert all(np.array_equal(a, b) for a, b in zip(_run(box, q, dt, variant=v), ref)), v
