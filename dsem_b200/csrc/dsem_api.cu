@@ -1543,7 +1543,7 @@ int shard_enqueue(dsem_ctx *c, double dt, int kk, int phase) {
     return fail(c, DSEM_ERR_INVALID_ARG, "stage index outside 1..kord or phase outside 0..2");
   long long l = 0;
   int r;
-  const unsigned nb = (unsigned)std::min<long long>(((long long)c->ncut * 5 * c->cut_G * c->cut_G + 255) / 256, 148LL * 8);
+  const unsigned nb = (unsigned)std::min<long long>(((long long)c->ncut * 5 * c->cut_G * c->cut_G + 255) / 256, 8LL * SM_COUNT);
   if (phase == 0) {  // stage start; local cut-face traces -> send
     if (!c->traces_valid && (r = enqueue_traces(c, &l))) return r;
     if (kk == 1) {

@@ -131,12 +131,7 @@ cudaError_t Launch<G>::vol(const VolArgs &a, int nel, bool diag, int mode, cudaS
 
 template <int G> cudaError_t Launch<G>::update(const UpdArgs &a, int nel, cudaStream_t s) {
   constexpr size_t smem = UPD_SMEM<G>;
-  static std::atomic<unsigned long long> attr[2] = {{0}, {0}};
-  if (smem > 48 * 1024) {
-    const cudaError_t e =
-        a.fmc ? set_smem_once(k_update<G, true>, smem, attr[1]) : set_smem_once(k_update<G, false>, smem, attr[0]);
-    if (e != cudaSuccess) return e;
-  }
+  static_assert(smem <= 48 * 1024, "more needs the kernel's shared-memory attribute");
   if (nel <= 0) return cudaSuccess;
   if (a.fmc)
     k_update<G, true><<<nel, 256, smem, s>>>(a);

@@ -806,7 +806,7 @@ static __global__ void __launch_bounds__(NC_THREADS) k_face_nc_vis(const MortarN
 struct VolArgs {
   const double *JQ;
   long long sq;
-  const double *jac, *gg, *gm;  // metrics, layout per DIAG
+  const double *jac, *gg, *gm;  // metrics: 3 arrays per element (diagonal) or 9 (full)
   const double *muhg;           // [elem][G^3] entropy viscosity (EV)
   const double *nuhg;           // [elem][G^3] Smagorinsky viscosity (LES; null: off)
   const double *QF;             // [elem][6][5][G^2] averaged face state
@@ -816,7 +816,6 @@ struct VolArgs {
   Phys P;
   const int *ecase;             // optional: case of each element (ensembles)
   const double *rec;            // optional: per case {re, 1/re}
-  int nel;                      // elements of the launch (set by the launcher)
 };
 
 // k_vol: full metrics (rotated, skewed or curved elements) at p = 1, 2, whose lines are too
