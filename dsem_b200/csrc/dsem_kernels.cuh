@@ -257,10 +257,11 @@ __device__ __forceinline__ void riemann(const double *nh, double ds, const doubl
 // Viscous fluxes (PhysLib.f90:419-583).  GX/GY/GZ hold the gradient
 // components of the five conserved variables (x, y, z derivatives).
 // The directional versions compute only what their flux vector reads.  MU: amu varies (a viscosity
-// model); else it is the constant 1 and so is the conductivity.  (A test of amu at run time diverges
-// where a model sets it on some points only: k_vol of 448 elements of p = 1 with entropy
-// viscosity 23.2 -> 24.1 us.)
-template <bool MU>
+// model); else it is the constant 1 and so is the conductivity.  TEST: a point's conductivity is
+// formed only where its amu is not 1, which diverges where a model acts on some points of a warp
+// (k_vol of 448 elements of p = 1 with entropy viscosity 23.2 -> 24.1 us, a step of 640 of p = 5 with
+// Smagorinsky's model 272.8 -> 282.1) but suits some launch shapes (VIS_TEST).
+template <bool MU, bool TEST = false>
 __device__ __forceinline__ void vis_flux_x(const double *Q, double rr, const double *Qx, const double *Qy,
                                            const double *Qz, double amu, const Phys &P, double *f) {
   const double gamma = P.gamma, gm1 = P.gm1;
@@ -272,7 +273,7 @@ __device__ __forceinline__ void vis_flux_x(const double *Q, double rr, const dou
   double wx = ddiv(Qx[3] - w * Qx[0], rho, rr), wz = ddiv(Qz[3] - w * Qz[0], rho, rr);
   double px = gm1 * (Qx[4] - 0.5 * Qx[0] * (u * u + v * v + w * w) - rho * (u * ux + v * vx + w * wx));
   double tx = ddiv((px - ddiv(p * Qx[0], rho, rr)) * P.mach * P.mach * gamma, rho, rr);
-  const double akappa = MU ? 1.0 + ddiv((amu - 1.0) * 2.0e-1, gm1, P.r_gm1) : 1.0;
+  const double akappa = !MU || (TEST && amu == 1.0) ? 1.0 : 1.0 + ddiv((amu - 1.0) * 2.0e-1, gm1, P.r_gm1);
   double div = ux + vy + wz;
   double sxy = uy + vx, sxz = wx + uz;
   f[0] = 0.0;
@@ -281,7 +282,7 @@ __device__ __forceinline__ void vis_flux_x(const double *Q, double rr, const dou
   f[3] = amu * sxz;
   f[4] = u * f[1] + v * f[2] + w * f[3] + ddiv(akappa * tx, P.den, P.r_den);
 }
-template <bool MU>
+template <bool MU, bool TEST = false>
 __device__ __forceinline__ void vis_flux_y(const double *Q, double rr, const double *Qx, const double *Qy,
                                            const double *Qz, double amu, const Phys &P, double *g) {
   const double gamma = P.gamma, gm1 = P.gm1;
@@ -293,7 +294,7 @@ __device__ __forceinline__ void vis_flux_y(const double *Q, double rr, const dou
   double wy = ddiv(Qy[3] - w * Qy[0], rho, rr), wz = ddiv(Qz[3] - w * Qz[0], rho, rr);
   double py = gm1 * (Qy[4] - 0.5 * Qy[0] * (u * u + v * v + w * w) - rho * (u * uy + v * vy + w * wy));
   double ty = ddiv((py - ddiv(p * Qy[0], rho, rr)) * P.mach * P.mach * gamma, rho, rr);
-  const double akappa = MU ? 1.0 + ddiv((amu - 1.0) * 2.0e-1, gm1, P.r_gm1) : 1.0;
+  const double akappa = !MU || (TEST && amu == 1.0) ? 1.0 : 1.0 + ddiv((amu - 1.0) * 2.0e-1, gm1, P.r_gm1);
   double div = ux + vy + wz;
   double sxy = uy + vx, syz = wy + vz;
   g[0] = 0.0;
@@ -302,7 +303,7 @@ __device__ __forceinline__ void vis_flux_y(const double *Q, double rr, const dou
   g[3] = amu * syz;
   g[4] = v * g[2] + u * g[1] + w * g[3] + ddiv(akappa * ty, P.den, P.r_den);
 }
-template <bool MU>
+template <bool MU, bool TEST = false>
 __device__ __forceinline__ void vis_flux_z(const double *Q, double rr, const double *Qx, const double *Qy,
                                            const double *Qz, double amu, const Phys &P, double *h) {
   const double gamma = P.gamma, gm1 = P.gm1;
@@ -314,7 +315,7 @@ __device__ __forceinline__ void vis_flux_z(const double *Q, double rr, const dou
   double wx = ddiv(Qx[3] - w * Qx[0], rho, rr), wy = ddiv(Qy[3] - w * Qy[0], rho, rr), wz = ddiv(Qz[3] - w * Qz[0], rho, rr);
   double pz = gm1 * (Qz[4] - 0.5 * Qz[0] * (u * u + v * v + w * w) - rho * (u * uz + v * vz + w * wz));
   double tz = ddiv((pz - ddiv(p * Qz[0], rho, rr)) * P.mach * P.mach * gamma, rho, rr);
-  const double akappa = MU ? 1.0 + ddiv((amu - 1.0) * 2.0e-1, gm1, P.r_gm1) : 1.0;
+  const double akappa = !MU || (TEST && amu == 1.0) ? 1.0 : 1.0 + ddiv((amu - 1.0) * 2.0e-1, gm1, P.r_gm1);
   double div = ux + vy + wz;
   double sxz = wx + uz, syz = wy + vz;
   h[0] = 0.0;

@@ -121,9 +121,17 @@ template <int G, int D> __device__ __forceinline__ constexpr int mma_stride() {
   return D == 0 ? 1 : (D == 1 ? G : mma_plane(G));
 }
 
+// Where k_vol_mma tests a point's viscosity (vis_flux_x): in the shapes whose register budget takes
+// that form better.  Steps, us, without / with the test: p = 6, 125 elements, Smagorinsky's model
+// 137.4 / 135.8; p = 7 wide, 64 elements, entropy viscosity 148.7 / 145.7; p = 8, 512 elements, the
+// same 574.6 / 566.1 (452 / 404 bytes of spills); the other way round p = 8 wide, 64 elements,
+// Smagorinsky's model 200.9 / 202.2, p = 7, 512 elements, the same 337.0 / 341.3, and p = 5.
+template <int G, int V>
+constexpr bool VIS_TEST = G == 7 || (G == 8 && V == MMA_WIDE) || (G == 9 && V != MMA_WIDE);
+
 // Viscous flux of direction D times gdiag into r from the point's state and its
 // 11 interpolated gradient fields (diag_field order).
-template <int D, bool MU>
+template <int D, bool MU, bool TEST>
 __device__ __forceinline__ void mma_vis(const double *Q, double rr, const double *c, double amu, double gdiag,
                                         const Phys &P, double *r) {
   double Qx[NV], Qy[NV], Qz[NV], fl[NV];
@@ -131,17 +139,17 @@ __device__ __forceinline__ void mma_vis(const double *Q, double rr, const double
     Qx[0] = c[0]; Qx[1] = c[1]; Qx[2] = c[2]; Qx[3] = c[3]; Qx[4] = c[4];
     Qy[0] = c[5]; Qy[1] = c[6]; Qy[2] = c[7]; Qy[3] = 0.0; Qy[4] = 0.0;
     Qz[0] = c[8]; Qz[1] = c[9]; Qz[3] = c[10]; Qz[2] = 0.0; Qz[4] = 0.0;
-    vis_flux_x<MU>(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_x<MU, TEST>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   } else if (D == 1) {
     Qy[0] = c[0]; Qy[1] = c[1]; Qy[2] = c[2]; Qy[3] = c[3]; Qy[4] = c[4];
     Qx[0] = c[5]; Qx[1] = c[6]; Qx[2] = c[7]; Qx[3] = 0.0; Qx[4] = 0.0;
     Qz[0] = c[8]; Qz[2] = c[9]; Qz[3] = c[10]; Qz[1] = 0.0; Qz[4] = 0.0;
-    vis_flux_y<MU>(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_y<MU, TEST>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   } else {
     Qz[0] = c[0]; Qz[1] = c[1]; Qz[2] = c[2]; Qz[3] = c[3]; Qz[4] = c[4];
     Qx[0] = c[5]; Qx[1] = c[6]; Qx[3] = c[7]; Qx[2] = 0.0; Qx[4] = 0.0;
     Qy[0] = c[8]; Qy[2] = c[9]; Qy[3] = c[10]; Qy[1] = 0.0; Qy[4] = 0.0;
-    vis_flux_z<MU>(Q, rr, Qx, Qy, Qz, amu, P, fl);
+    vis_flux_z<MU, TEST>(Q, rr, Qx, Qy, Qz, amu, P, fl);
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) r[v] = gdiag * fl[v];
@@ -295,7 +303,7 @@ __device__ __forceinline__ void mma_tile(int t, const MmaOps<G, V> &O, const Phy
     if (ev) amu = amu + mu[i];
     const double rr = 1.0 / Q[i][0];
     double r[NV], fi[NV];
-    mma_vis<D, MU>(Q[i], rr, c[i], amu, gd[i], P, r);
+    mma_vis<D, MU, VIS_TEST<G, V>>(Q[i], rr, c[i], amu, gd[i], P, r);
     euler_flux(D, Q[i], rr, P.gm1, fi);
     const bool in = (i == 0 ? 1 : 5) + q <= C::NS;  // padded points contribute exact zeros
 #pragma unroll
@@ -349,7 +357,7 @@ __device__ __forceinline__ void mma_faces(int ln, const Phys &P, const double *Q
     double amu = 1.0;
     if (les) amu = amu + nu[i] * Q[i][0];
     if (ev) amu = amu + mu[i];
-    mma_vis<D, MU>(Q[i], 1.0 / Q[i][0], c[i], amu, gd[i], P, r);
+    mma_vis<D, MU, VIS_TEST<G, V>>(Q[i], 1.0 / Q[i][0], c[i], amu, gd[i], P, r);
     double *o = VF + ((i ? face_hi(D) : face_lo(D)) - 1) * 5 * G2 + ln;
 #pragma unroll
     for (int v = 0; v < NV; ++v) o[v * G2] = r[v];
@@ -538,10 +546,11 @@ __global__ void __launch_bounds__(MmaCfg<G, V>::NT, MmaCfg<G, V>::MINB) k_vol_mm
 // k_vol_mma_gen: the same for elements with full metrics (rotated, skewed or curved), all
 // 15 gradient components kept (k_vol's sums over the directions x, y, z) and all three
 // fluxes formed at every point.  Bound by the FP64 pipe like the diagonal kernel, with about
-// twice its work.  20 shared fields: one element per SM at p >= 7, so 12 warps (168
-// registers) per element.  Measured, ms per volume launch, k_vol -> this: 10^3 curved
+// twice its work.  20 shared fields: two elements fit an SM's shared memory at p = 7 (87 KB
+// each), one at p = 8 (121 KB); the 12 warps of 168 registers take one element per SM at both.  Measured, ms per volume launch, k_vol -> this: 10^3 curved
 // elements of p = 8 0.415 -> 0.218, p = 7 0.253 -> 0.137, 12^3 of p = 6 0.281 -> 0.171,
 // p = 5 0.169 -> 0.128, 14^3 of p = 4 0.213 -> 0.098, p = 3 0.089 -> 0.048.
+
 // Contributions of the derivative along D to the Gauss gradients of the five fields on a
 // tile's lines (Gauss_Deriv, SolnDerivsc.f90:36-80): stored for D = 0, added after.
 template <int G, int V, int D>
