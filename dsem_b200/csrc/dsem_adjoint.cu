@@ -62,28 +62,30 @@ struct AdjBuf {
   double *evb_prev = nullptr;
   double *lrb = nullptr;  // boundary faces: per boundary point, dJ/d(1/Re) of the external viscous flux
   double *volscr = nullptr;  // p = 7, 8: the volume adjoint's per element scratch (VolAdjCfg::SCR)
-  // Device memory: one block for all buffers of the call, or, when that cannot be had, a
-  // cudaMalloc per buffer, so that the optional ones can fail one by one.  Measured for 18
-  // buffers of 2.25 GB together (8^3 elements of p = 6, 30 steps, every stage kept): 18 x
-  // (cudaMalloc + cudaFree) 13.8 ms and now and then 290; one pair 2.5.  A stream-ordered pool
-  // maps and unmaps by the byte: 28 ms for its first use and its end, 0.04 between them; at
-  // 0.3 GB 3.9 against 11 and 0.9.  So a block of at most ADJ_POOL_KEEP comes from the
-  // context's pool, which keeps it for the next call (the driver takes it back when another
-  // allocation needs the memory), and a larger one is mapped and freed by the call.
+  // Device memory: one block for all buffers of the call, which the context keeps for its next
+  // one, or, when that cannot be had, a cudaMalloc per buffer, so that the optional ones can fail
+  // one by one.  Measured for 18 buffers of 2.25 GB together (8^3 elements of p = 6, 30 steps, every
+  // stage kept): 18 x (cudaMalloc + cudaFree) 13.8 ms and now and then 290; one pair 2.5 (8 GB: 17.6
+  // and 6.8).  A stream-ordered pool maps and unmaps by the byte: 28 ms for its first use and
+  // its end, and 48 in every call at 8 GB when it keeps less.
   dsem_ctx *c = nullptr;
   char *block = nullptr;
   size_t size = 0, used = 0;
-  bool pooled = false;
   std::vector<double *> own;  // buffers with a cudaMalloc of their own
   static size_t padded(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
-  void reserve(size_t bytes);
+  void reserve(size_t bytes) {
+    void *p = dsem_int::block_take(c, bytes, &size);
+    if (!p && dsem_int::dev_malloc(&p, bytes) == cudaSuccess) size = bytes;
+    cudaGetLastError();
+    block = static_cast<char *>(p);
+  }
   cudaError_t alloc(double **p, size_t bytes) {
     if (block && padded(bytes) <= size - used) {
       *p = reinterpret_cast<double *>(block + used);
       used += padded(bytes);
       return cudaSuccess;
     }
-    const cudaError_t e = cudaMalloc(p, bytes);
+    const cudaError_t e = dsem_int::dev_malloc(p, bytes);
     if (e == cudaSuccess) own.push_back(*p);
     return e;
   }
@@ -97,43 +99,9 @@ struct AdjBuf {
   }
   ~AdjBuf() {
     for (double *p : own) cudaFree(p);
-    if (pooled) {
-      cudaFreeAsync(block, c->st);
-      cudaStreamSynchronize(c->st);  // what the pool does not keep is given back here
-    } else {
-      cudaFree(block);
-    }
+    dsem_int::block_give(c, block, size);  // (the next call's work follows on the same stream)
   }
 };
-
-// The pool of the smaller blocks, made by the first call that needs it and destroyed with the
-// context.  It keeps at most ADJ_POOL_KEEP bytes between calls: 256 MiB, below which its first
-// use and its end together still take less than the separate allocations did.
-constexpr size_t ADJ_POOL_KEEP = (size_t)256 << 20;
-bool adj_pool(dsem_ctx *c) {
-  if (c->adj_pool) return true;
-  cudaMemPoolProps props{};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = c->dev;
-  unsigned long long keep = ADJ_POOL_KEEP;
-  if (cudaMemPoolCreate(&c->adj_pool, &props) != cudaSuccess) {
-    c->adj_pool = nullptr;
-    return false;
-  }
-  return cudaMemPoolSetAttribute(c->adj_pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
-}
-
-void AdjBuf::reserve(size_t bytes) {
-  void *p = nullptr;
-  if (bytes <= ADJ_POOL_KEEP)
-    pooled = adj_pool(c) && cudaMallocFromPoolAsync(&p, bytes, c->adj_pool, c->st) == cudaSuccess;
-  if (pooled || cudaMalloc(&p, bytes) == cudaSuccess) {
-    block = static_cast<char *>(p);
-    size = bytes;
-  }
-  cudaGetLastError();
-}
 
 // Where a group's slices of the adjoint's buffers start (doubles, or elements for e0)
 struct GOff {

@@ -528,7 +528,7 @@ int ensure_stage_buf(dsem_ctx *c, int ldx, int nf) {
   if (need > c->nstage) {
     if (c->stage) cudaFree(c->stage);
     c->stage = nullptr;
-    CK(cudaMalloc(&c->stage, need * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->stage, need * sizeof(double)));
     c->nstage = need;
   }
   return DSEM_OK;
@@ -819,25 +819,25 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
             }
       }
     }
-    CK(cudaMalloc(&g.jac, jac.size() * sizeof(double)));
-    CK(cudaMalloc(&g.hd, hd.size() * sizeof(double)));
-    CK(cudaMalloc(&g.gg, gg.size() * sizeof(double)));
-    CK(cudaMalloc(&g.gm, gmv.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.jac, jac.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.hd, hd.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.gg, gg.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.gm, gmv.size() * sizeof(double)));
     CK(cudaMemcpy(g.jac, jac.data(), jac.size() * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.hd, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.gg, gg.data(), gg.size() * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.gm, gmv.data(), gmv.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&g.muhg, (size_t)g.nel * NG * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.muhg, (size_t)g.nel * NG * sizeof(double)));
     CK(cudaMemset(g.muhg, 0, (size_t)g.nel * NG * sizeof(double)));
-    CK(cudaMalloc(&g.EVB, (size_t)g.nel * 15 * NG * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.EVB, (size_t)g.nel * 15 * NG * sizeof(double)));
     CK(cudaMemset(g.EVB, 0, (size_t)g.nel * 15 * NG * sizeof(double)));
-    CK(cudaMalloc(&g.int2ext, ids.size() * sizeof(int)));
+    CK(dsem_int::dev_malloc(&g.int2ext, ids.size() * sizeof(int)));
     CK(cudaMemcpy(g.int2ext, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&g.ecase, ec.size() * sizeof(int)));
+    CK(dsem_int::dev_malloc(&g.ecase, ec.size() * sizeof(int)));
     CK(cudaMemcpy(g.ecase, ec.data(), ec.size() * sizeof(int), cudaMemcpyHostToDevice));
     std::vector<double> kw(NG);
     hostmath::ke_weights(G, kw.data());
-    CK(cudaMalloc(&g.kew, NG * sizeof(double)));
+    CK(dsem_int::dev_malloc(&g.kew, NG * sizeof(double)));
     CK(cudaMemcpy(g.kew, kw.data(), NG * sizeof(double), cudaMemcpyHostToDevice));
     c->groups.push_back(g);
     q0 += 5LL * g.nel * NG;
@@ -1005,11 +1005,11 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
     MList ml;
     ml.G = G;
     ml.n = (int)mcs[G].size();
-    CK(cudaMalloc(&ml.mc, mcs[G].size() * sizeof(MortarC)));
+    CK(dsem_int::dev_malloc(&ml.mc, mcs[G].size() * sizeof(MortarC)));
     CK(cudaMemcpy(ml.mc, mcs[G].data(), mcs[G].size() * sizeof(MortarC), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&ml.nh, nhs[G].size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&ml.nh, nhs[G].size() * sizeof(double)));
     CK(cudaMemcpy(ml.nh, nhs[G].data(), nhs[G].size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&ml.nrm, nrs[G].size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&ml.nrm, nrs[G].size() * sizeof(double)));
     CK(cudaMemcpy(ml.nrm, nrs[G].data(), nrs[G].size() * sizeof(double), cudaMemcpyHostToDevice));
     c->mlists.push_back(ml);
   }
@@ -1020,15 +1020,15 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
     bl.n = (int)bms[G].size();
     bl.mortar = bids[G];
     const size_t next = (size_t)bl.n * 5 * G * G;
-    CK(cudaMalloc(&bl.mb, bms[G].size() * sizeof(dsem::MortarB)));
+    CK(dsem_int::dev_malloc(&bl.mb, bms[G].size() * sizeof(dsem::MortarB)));
     CK(cudaMemcpy(bl.mb, bms[G].data(), bms[G].size() * sizeof(dsem::MortarB), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&bl.nh, bnhs[G].size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&bl.nh, bnhs[G].size() * sizeof(double)));
     CK(cudaMemcpy(bl.nh, bnhs[G].data(), bnhs[G].size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&bl.nrm, bnrs[G].size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&bl.nrm, bnrs[G].size() * sizeof(double)));
     CK(cudaMemcpy(bl.nrm, bnrs[G].data(), bnrs[G].size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&bl.qext, next * sizeof(double)));
+    CK(dsem_int::dev_malloc(&bl.qext, next * sizeof(double)));
     CK(cudaMemset(bl.qext, 0, next * sizeof(double)));
-    CK(cudaMalloc(&bl.fvext, next * sizeof(double)));
+    CK(dsem_int::dev_malloc(&bl.fvext, next * sizeof(double)));
     CK(cudaMemset(bl.fvext, 0, next * sizeof(double)));
     c->nbnd += bl.n;
     c->blists.push_back(bl);
@@ -1044,30 +1044,30 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
     }
     c->ncut = n;
     c->cut_G = cut_G;
-    CK(cudaMalloc(&c->cut, n * sizeof(MortarCut)));
+    CK(dsem_int::dev_malloc(&c->cut, n * sizeof(MortarCut)));
     CK(cudaMemcpy(c->cut, cuts.data(), n * sizeof(MortarCut), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->cut_nh, cut_nh.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->cut_nh, cut_nh.size() * sizeof(double)));
     CK(cudaMemcpy(c->cut_nh, cut_nh.data(), cut_nh.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->cut_nrm, cut_nrm.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->cut_nrm, cut_nrm.size() * sizeof(double)));
     CK(cudaMemcpy(c->cut_nrm, cut_nrm.data(), cut_nrm.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->pack_src, n * sizeof(long long)));
+    CK(dsem_int::dev_malloc(&c->pack_src, n * sizeof(long long)));
     CK(cudaMemcpy(c->pack_src, src.data(), n * sizeof(long long), cudaMemcpyHostToDevice));
     const size_t nb = (size_t)n * 5 * cut_G * cut_G * sizeof(double);
-    CK(cudaMalloc(&c->send, nb));
-    CK(cudaMalloc(&c->ghost, nb));
+    CK(dsem_int::dev_malloc(&c->send, nb));
+    CK(dsem_int::dev_malloc(&c->ghost, nb));
     CK(cudaMemset(c->send, 0, nb));
     CK(cudaMemset(c->ghost, 0, nb));
   }
 
   if (!ncs.empty()) {
     c->nnc = (int)ncs.size();
-    CK(cudaMalloc(&c->nc, ncs.size() * sizeof(MortarNC)));
+    CK(dsem_int::dev_malloc(&c->nc, ncs.size() * sizeof(MortarNC)));
     CK(cudaMemcpy(c->nc, ncs.data(), ncs.size() * sizeof(MortarNC), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->nc_nh, nc_nh.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->nc_nh, nc_nh.size() * sizeof(double)));
     CK(cudaMemcpy(c->nc_nh, nc_nh.data(), nc_nh.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->nc_nrm, nc_nrm.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->nc_nrm, nc_nrm.size() * sizeof(double)));
     CK(cudaMemcpy(c->nc_nrm, nc_nrm.data(), nc_nrm.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->nc_mats, std::max<size_t>(1, mats.size()) * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->nc_mats, std::max<size_t>(1, mats.size()) * sizeof(double)));
     if (!mats.empty()) CK(cudaMemcpy(c->nc_mats, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
   }
 
@@ -1109,7 +1109,7 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
     if (ok) {
       for (size_t gi = 0; gi < ng; ++gi) {
         Group &g = c->groups[gi];
-        CK(cudaMalloc(&g.fmc, fm[gi].size() * sizeof(MortarC)));
+        CK(dsem_int::dev_malloc(&g.fmc, fm[gi].size() * sizeof(MortarC)));
         CK(cudaMemcpy(g.fmc, fm[gi].data(), fm[gi].size() * sizeof(MortarC), cudaMemcpyHostToDevice));
       }
       c->fuse_vis = true;
@@ -1117,17 +1117,17 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
   }
 
   // ---- state and face buffers
-  CK(cudaMalloc(&c->JQ, c->nq * sizeof(double)));
-  CK(cudaMalloc(&c->gQ, c->nq * sizeof(double)));
-  CK(cudaMalloc(&c->QTI, c->nq * sizeof(double)));
-  CK(cudaMalloc(&c->Qt, c->nq * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->JQ, c->nq * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->gQ, c->nq * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->QTI, c->nq * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->Qt, c->nq * sizeof(double)));
   CK(cudaMemset(c->JQ, 0, c->nq * sizeof(double)));
   CK(cudaMemset(c->gQ, 0, c->nq * sizeof(double)));
-  CK(cudaMalloc(&c->QF, c->nface * sizeof(double)));
-  CK(cudaMalloc(&c->FF, c->nface * sizeof(double)));
-  CK(cudaMalloc(&c->VF, c->nface * sizeof(double)));
-  CK(cudaMalloc(&c->part, (size_t)ngrid * 5 * sizeof(double)));
-  CK(cudaMalloc(&c->flag, sizeof(int)));
+  CK(dsem_int::dev_malloc(&c->QF, c->nface * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->FF, c->nface * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->VF, c->nface * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->part, (size_t)ngrid * 5 * sizeof(double)));
+  CK(dsem_int::dev_malloc(&c->flag, sizeof(int)));
   CK(cudaMemset(c->flag, 0, sizeof(int)));
   CK(cudaEventCreate(&c->e0));
   CK(cudaEventCreate(&c->e1));
@@ -1138,9 +1138,9 @@ int setup_ctx(dsem_ctx *c, const MeshSet &ms) {
       rec[2 * k] = c->case_re[k];
       rec[2 * k + 1] = 1.0 / c->case_re[k];
     }
-    CK(cudaMalloc(&c->d_rec, rec.size() * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->d_rec, rec.size() * sizeof(double)));
     CK(cudaMemcpy(c->d_rec, rec.data(), rec.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->d_dtc, (size_t)c->ncase * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->d_dtc, (size_t)c->ncase * sizeof(double)));
     CK(cudaMemset(c->d_dtc, 0, (size_t)c->ncase * sizeof(double)));
   }
   // streams for the parallel branches of a stage
@@ -1223,7 +1223,7 @@ void dsem_destroy(dsem_ctx *c) {
   cudaFree(c->flag);
   if (c->e0) cudaEventDestroy(c->e0);
   if (c->e1) cudaEventDestroy(c->e1);
-  if (c->adj_pool) cudaMemPoolDestroy(c->adj_pool);
+  dsem_int::block_drop(c);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
@@ -1424,7 +1424,7 @@ int dsem_keep_lobatto(dsem_ctx *c, int on) {
       g.l0 = n;
       n += (long long)g.nel * 15 * (g.G + 1) * g.G * g.G;
     }
-    CK(cudaMalloc(&c->QLB, (size_t)std::max(n, 1LL) * sizeof(double)));
+    CK(dsem_int::dev_malloc(&c->QLB, (size_t)std::max(n, 1LL) * sizeof(double)));
   }
   c->keep_lob = on != 0;
   c->lob_valid = false;
@@ -1729,7 +1729,7 @@ int dsem_set_les(dsem_ctx *c, double cs, double numax) {
     for (auto &g : c->groups) {
       if (!g.nuhg) {
         const size_t n = (size_t)g.nel * g.G * g.G * g.G;
-        CK(cudaMalloc(&g.nuhg, n * sizeof(double)));
+        CK(dsem_int::dev_malloc(&g.nuhg, n * sizeof(double)));
         CK(cudaMemset(g.nuhg, 0, n * sizeof(double)));
       }
     }
@@ -1751,7 +1751,7 @@ int dsem_set_les_sensors(dsem_ctx *c, int shock_sensor, int rho_sensor) {
     for (auto &g : c->groups) {
       if (!g.sens) {
         const size_t n = (size_t)g.nel * 2 * g.G * g.G * g.G;
-        CK(cudaMalloc(&g.sens, n * sizeof(double)));
+        CK(dsem_int::dev_malloc(&g.sens, n * sizeof(double)));
         CK(cudaMemset(g.sens, 0, n * sizeof(double)));
       }
     }

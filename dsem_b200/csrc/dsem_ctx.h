@@ -104,7 +104,6 @@ struct dsem_ctx {
   bool keep_lob = false;  // the last stage of every step stores them (dsem_keep_lobatto)
   bool lob_valid = false; // QLB holds the arrays of the last stage run
   int adj_scheme = 0;     // dsem_adjoint with snapshots > 0: DSEM_ADJ_REVOLVE or DSEM_ADJ_SEGMENTS
-  cudaMemPool_t adj_pool = nullptr;  // dsem_adjoint's buffers when they are small
   cudaGraphExec_t gexec = nullptr;
   int graph_key = -1;
   long long graph_launches = 0;
@@ -139,6 +138,17 @@ void dsem_set_thread_error(const std::string &msg);
 // Internal entry points of the API translation unit used by the adjoint.
 namespace dsem_int {
 int fail(dsem_ctx *c, int code, const std::string &msg);
+// The device block that a context keeps for its next dsem_adjoint (dsem_blocks.cu)
+void *block_take(const dsem_ctx *c, size_t bytes, size_t *size);  // one of at least bytes, or null (a smaller one is freed)
+void block_give(const dsem_ctx *c, void *p, size_t size);         // keeps it, or frees it (BLOCK_MAX, BLOCK_KEEP)
+bool block_drop(const dsem_ctx *c);                               // frees c's (null: every context's); false: there was none
+// cudaMalloc for everything the library allocates: takes back the kept blocks before it fails
+template <class T> cudaError_t dev_malloc(T **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !block_drop(nullptr)) return e;
+  cudaGetLastError();
+  return cudaMalloc(p, bytes);
+}
 int stage(dsem_ctx *c, int kk, bool save);  // one RK stage on c->JQ (eager launches)
 int traces(dsem_ctx *c);                    // face traces of c->JQ
 int ev(dsem_ctx *c, const double *jq = nullptr);  // entropy viscosity of jq (null: c->JQ; valid: c->ev_grad_valid)

@@ -311,9 +311,10 @@ int dsem_diag_batch(dsem_ctx *ctx, const double *dt, int first, double *ke, doub
  * each snapshot also keeps the gradients its step's viscosity reads),
  * boundary faces of every kind (walls, inflow, outflow; with them
  * DSEM_ADJ_SEGMENTS falls back to revolve), no sharding
- * (DSEM_ERR_UNSUPPORTED otherwise).  A call that needs at most 256 MiB of
- * device memory leaves it with the context for the next one (dsem_destroy
- * gives it back); a larger call frees what it allocated. */
+ * (DSEM_ERR_UNSUPPORTED otherwise).  The context keeps the call's device
+ * memory for its next one up to 4 GiB, all contexts together up to 16 GiB (a
+ * call that would exceed either frees it); dsem_destroy gives it back, and so
+ * does any later allocation of the library that would fail otherwise. */
 int dsem_adjoint(dsem_ctx *ctx, double dt, int nsteps, int window, int snapshots, double *J, double *dJdQ0,
                  int ldx, double *dJdinvRe, double *ms);
 
