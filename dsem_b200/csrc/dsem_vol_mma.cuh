@@ -31,7 +31,7 @@
 //
 // Measured (22^3 elements of p = 8, the volume launch): 1.757 -> 1.127 ms; p = 7,
 // 20^3: 1.286 -> 0.492; p = 6, 24^3: 1.088 -> 0.745; p = 5, 24^3: 0.568 -> 0.526;
-// p = 4, 32^3: 0.716 -> 0.640; p = 3, 32^3: 0.371 -> 0.299.
+// p = 4, 32^3: 0.717 -> 0.638; p = 3, 32^3: 0.372 -> 0.310.
 #pragma once
 #include "dsem_shapes.h"
 #include "dsem_stage.cuh"
@@ -548,8 +548,8 @@ __global__ void __launch_bounds__(MmaCfg<G, V>::NT, MmaCfg<G, V>::MINB) k_vol_mm
 // fluxes formed at every point.  Bound by the FP64 pipe like the diagonal kernel, with about
 // twice its work.  20 shared fields: two elements fit an SM's shared memory at p = 7 (87 KB
 // each), one at p = 8 (121 KB); the 12 warps of 168 registers take one element per SM at both.  Measured, ms per volume launch, k_vol -> this: 10^3 curved
-// elements of p = 8 0.415 -> 0.218, p = 7 0.253 -> 0.137, 12^3 of p = 6 0.281 -> 0.171,
-// p = 5 0.169 -> 0.128, 14^3 of p = 4 0.213 -> 0.098, p = 3 0.089 -> 0.048.
+// elements of p = 8 0.414 -> 0.217, p = 7 0.252 -> 0.135, 12^3 of p = 6 0.280 -> 0.169,
+// p = 5 0.168 -> 0.124, 14^3 of p = 4 0.212 -> 0.096, p = 3 0.090 -> 0.047.
 
 // Contributions of the derivative along D to the Gauss gradients of the five fields on a
 // tile's lines (Gauss_Deriv, SolnDerivsc.f90:36-80): stored for D = 0, added after.
